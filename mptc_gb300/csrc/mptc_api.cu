@@ -320,6 +320,39 @@ int launch_intra_sweeps(const mptc::SearchParams &P, const uint32_t *pending, co
   return sweeps + 1;
 }
 
+// The intra search of a whole intra frame (P.done zeroed): the row pipeline on
+// `ctas` SMs at sa <= 8 (after the weight sums of the stb words it reads), the
+// block dataflow on `grid` CTAs for larger windows. Returns the number of
+// kernels launched.
+int launch_intra_frame(const mptc::SearchParams &P, float4 *wdesc, const uint32_t *order, int grid, int ctas,
+                       cudaStream_t s) {
+  const int nblk = P.bw * P.bh;
+  if (P.sa > 8) {
+    mptc::intra_search_kernel<kIntraThreads><<<grid, kIntraThreads, 0, s>>>(P, order, nullptr, nblk);
+    return 1;
+  }
+  mptc::weight_desc_kernel<<<(nblk + 255) / 256, 256, 0, s>>>(P.stb, nblk, wdesc);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(mptc::kRowCluster * std::max(1, std::min(P.bh, ctas / mptc::kRowCluster)));
+  cfg.blockDim = dim3(mptc::kRowThreads);
+  cfg.dynamicSmemBytes = sizeof(mptc::RowShared);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = mptc::kRowCluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, mptc::intra_rows_kernel, P);
+  return 2;
+}
+
+// The row pipeline's shared memory (its warps' tables).
+cudaError_t intra_rows_attr() {
+  return cudaFuncSetAttribute(mptc::intra_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(mptc::RowShared));
+}
+
 // The exhaustive inter search: one warp per run of kInterRun blocks of a row
 // at sa <= 8 (the runs share the deduplication of their windows; a persistent
 // grid of 32 warps per SM takes the runs from the zeroed counter work[7]),
@@ -604,8 +637,9 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
                                            sweep_count(ctx->cfg.intra_sweeps), ctx->sweep_part,
                                            std::min(ctx->nblk, kSweepPartCap), s);
     else
-      mptc::intra_search_kernel<kIntraThreads><<<ig, kIntraThreads, 0, s>>>(P, ctx->order, nullptr, ctx->nblk);
-    if (!prev_final_dev) ++ctx->launches;
+      ctx->launches += launch_intra_frame(P, ctx->wdesc, ctx->order, ig,
+                                          ctx->intra_cap > 0 ? std::min(ctx->intra_cap, ctx->sm_count) : ctx->sm_count,
+                                          s);
   }
   MPTC_CUDA(cudaGetLastError());
   const uint16_t *m16 = P.motion;
@@ -661,7 +695,7 @@ mptc_status mptc_ctx_create(const mptc_config *cfg, int32_t width, int32_t heigh
   if (cudaGetDevice(&ctx->device) != cudaSuccess) return bad(MPTC_ECUDA);
   if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess)
     return bad(MPTC_ECUDA);
-  if (ensure_tables(ctx->device) != cudaSuccess) return bad(MPTC_ECUDA);
+  if (ensure_tables(ctx->device) != cudaSuccess || intra_rows_attr() != cudaSuccess) return bad(MPTC_ECUDA);
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mptc::intra_search_kernel<kIntraThreads>,
                                                     kIntraThreads, 0) != cudaSuccess)
@@ -1344,7 +1378,7 @@ mptc_status noalloc_setup(int device, NoallocDevice **out) {
   if (!d.ready) {
     void *p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return MPTC_ECUDA;
-    if (ensure_tables(device) != cudaSuccess) return MPTC_ECUDA;
+    if (ensure_tables(device) != cudaSuccess || intra_rows_attr() != cudaSuccess) return MPTC_ECUDA;
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return MPTC_ECUDA;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mptc::intra_search_kernel<kIntraThreads>,
@@ -1431,7 +1465,7 @@ extern "C" mptc_status mptc_encode_frame_noalloc(const mptc_config *cfg, int32_t
                                                     work + 1);
     launch_intra_sweeps(P, pend, work + 5, sweep, n, d->intra_grid, sw, sweep_part, kSweepPartCapNoalloc, s);
   } else {
-    mptc::intra_search_kernel<kIntraThreads><<<d->intra_grid, kIntraThreads, 0, s>>>(P, order, nullptr, n);
+    launch_intra_frame(P, wdesc, order, d->intra_grid, d->sm_count, s);
   }
   const uint16_t *m16 = reinterpret_cast<const uint16_t *>(motion_dev);
   mptc::unique_scan_kernel<<<ntiles, 256, 0, s>>>(m16, stb, n, ntiles, tile_state + ntiles, work + 11, unique_dev,

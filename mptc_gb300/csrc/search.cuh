@@ -24,5 +24,6 @@
 #include "selection.cuh"
 #include "completion.cuh"
 #include "inter_search.cuh"
+#include "intra_rows.cuh"
 #include "intra_search.cuh"
 #include "scan.cuh"
