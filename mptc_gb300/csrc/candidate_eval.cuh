@@ -277,4 +277,164 @@ __device__ __forceinline__ int eval_candidate(const BlockTab &t, const PixelGrou
   return (int)((uint32_t)sse / 48u) - orig_err;
 }
 
+// ---- the same evaluation from integer sums --------------------------------------
+// The refit's inputs are small integers: with order o = {0, 3, 1, 2}[index] the
+// sums are bx = S / 3 and ax = (3 T - S) / 3, S = sum px * o (four dp4a per
+// channel) and T = sum px. The reference accumulates px * a and px * b in float,
+// pixel by pixel; its rounding only matters where the refitted endpoint + 0.5
+// falls next to an integer at which the snapped value changes. So the endpoints
+// are computed from the exact sums and the candidate is decided where all six
+// keep clear of such an integer by more than the two computations can differ; the
+// others (ties in the small rational grid of the endpoints, mostly: about 1% of
+// the candidates on the test streams) go through the reference's own float steps
+// (refit_exact).
+//
+// Bound: with u = 2^-24, 16 terms of relative error <= 2u (px * fl(1/3)) added in
+// 15 roundings give ax, bx to 17.1u; here each sum is one product (2u). The two
+// products, their difference and the products with the weight sums' float values
+// (the same in both) add 4u of ax * bsq + bx * ab, which is at most
+// T * max(asq, bsq): |difference| <= 23.1u * |f| * T * max(asq, bsq) + 5u * |p| plus
+// the two roundings of p + 0.5 (each <= 2^-17). |p| <= 260 covers every value that
+// the clamp to [0, 255] leaves. Where that is not below a half (a degenerate
+// word, all indices equal: f huge, infinite or NaN), refit_exact decides.
+constexpr float kRefitRel = 1.46e-6f;  // > 23.1u (1.05 x)
+constexpr float kRefitAbs = 1.0e-4f;   // > 260 * 5u + 2^-16
+
+struct __align__(16) PixBlock {
+  uint32_t pg[3][4];  // channel c bytes of pixels 4g .. 4g+3
+  uint32_t sum[3];    // sum of channel c
+  uint32_t sumsq;     // sum of squares over all channels
+};
+
+// The snap tables with, per value, whether the snapped value differs from that
+// of the value before (bit 31) and after (bit 30); the snapped value in the low
+// byte.
+constexpr uint32_t kSnapLow = 0x80000000u, kSnapHigh = 0x40000000u;
+struct SnapTables {
+  uint32_t five[256], six[256];
+};
+__device__ __forceinline__ void build_snap_edges(SnapTables &t) {
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+    const uint32_t x = (uint32_t)i & 255u, keep = i < 256 ? 0xF8u : 0xFCu, step = i < 256 ? 4u : 2u, sh = i < 256 ? 5u : 6u;
+    uint32_t v = snap_value(x, keep, step, sh);
+    const uint32_t lo = x > 0u ? snap_value(x - 1u, keep, step, sh) : v, hi = x < 255u ? snap_value(x + 1u, keep, step, sh) : v;
+    const uint32_t e = v | (lo != v ? kSnapLow : 0u) | (hi != v ? kSnapHigh : 0u);
+    (i < 256 ? t.five : t.six)[x] = e;
+  }
+}
+
+// The channel words (bytes of pixels 0 .. 3) of pixel row y of block column bx:
+// three aligned words of the frame (rows and blocks are a multiple of 4 bytes
+// apart).
+__device__ __forceinline__ void load_channels(const uint8_t *__restrict__ rgb, int width, int bx, int y, uint32_t &c0,
+                                              uint32_t &c1, uint32_t &c2) {
+  const uint32_t *p = reinterpret_cast<const uint32_t *>(rgb + ((size_t)y * width + 4 * bx) * 3);
+  const uint32_t w0 = __ldg(p), w1 = __ldg(p + 1), w2 = __ldg(p + 2);  // R0G0B0R1 G1B1R2G2 B2R3G3B3
+  c0 = __byte_perm(__byte_perm(w0, w1, 0x0630), w2, 0x5210);
+  c1 = __byte_perm(__byte_perm(w0, w1, 0x0741), w2, 0x6210);
+  c2 = __byte_perm(__byte_perm(w0, w1, 0x0052), w2, 0x7410);
+}
+
+// A refit's six endpoint values as entries of the snap tables: ep1's r, g, b, then
+// ep2's.
+struct RefitValues {
+  uint32_t snap[6];
+};
+
+// From the exact sums; false where the float steps may give another value.
+__device__ __forceinline__ bool refit_quick(const PixBlock &t, const SnapTables &st, uint32_t cand,
+                                            const WeightSums &ws, RefitValues &r) {
+  const float third = __fdiv_rn(1.0f, 3.0f);
+  uint32_t ord[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) ord[g] = __byte_perm(0x02010300u, 0u, spread_nibbles((cand >> (8 * g)) & 0xFFu));
+  const float tmax = __uint2float_rn(max(t.sum[0], max(t.sum[1], t.sum[2])));
+  const float margin =
+      __fmaf_rn(__fmul_rn(__fmul_rn(kRefitRel, tmax), fabsf(ws.f)), fmaxf(ws.asq, ws.bsq), kRefitAbs);
+  uint32_t edge = 0;  // bit 31: a value within the margin of an integer where its snapped value changes
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    uint32_t S = 0;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) S = __dp4a(t.pg[c][g], ord[g], S);
+    const float b = __fmul_rn(__uint2float_rn(S), third), a = __fmul_rn(__uint2float_rn(3u * t.sum[c] - S), third);
+    const float v1 = __fmaf_rn(ws.f, __fsub_rn(__fmul_rn(a, ws.bsq), __fmul_rn(b, ws.ab)), 0.5f);
+    const float v2 = __fmaf_rn(ws.f, __fsub_rn(__fmul_rn(b, ws.asq), __fmul_rn(a, ws.ab)), 0.5f);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float w = fminf(fmaxf(h ? v2 : v1, 0.5f), 255.5f);
+      const float m = __fadd_rd(w, 8388608.0f);  // floor(w) in the low bits
+      const float frac = __fsub_rn(w, __fsub_rn(m, 8388608.0f));
+      const uint32_t e = (c == 1 ? st.six : st.five)[__float_as_uint(m) & 0xFFu];
+      edge |= (__float_as_uint(__fsub_rn(frac, margin)) & e) |
+              (__float_as_uint(__fsub_rn(__fsub_rn(1.0f, margin), frac)) & (e << 1));
+      r.snap[3 * h + c] = e;
+    }
+  }
+  return (int)edge >= 0 && margin < 0.5f;  // false for a NaN or infinite margin
+}
+
+// By the reference's own steps (codec/dxt_image.cpp:298-331).
+__device__ __forceinline__ void refit_exact(const PixBlock &t, const SnapTables &st, uint32_t cand,
+                                            const WeightSums &ws, RefitValues &r) {
+  const float third = __fdiv_rn(1.0f, 3.0f), third2 = __fadd_rn(third, third);
+  float ax[3] = {0.f, 0.f, 0.f}, bx[3] = {0.f, 0.f, 0.f};
+#pragma unroll 1
+  for (int g = 0; g < 4; ++g) {
+    const uint32_t w[3] = {t.pg[0][g], t.pg[1][g], t.pg[2][g]}, idx = cand >> (8 * g);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t k = (idx >> (2 * i)) & 3u;
+      // px * a, px * b of the index: (1, 0), (0, 1), (2/3, 1/3), (1/3, 2/3)
+      const float lo = (k & 2u) ? third2 : 1.0f, hi = (k & 2u) ? third : 0.0f;
+      const float fa = (k & 1u) ? hi : lo, fb = (k & 1u) ? lo : hi;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float px = __uint2float_rn((w[c] >> (8 * i)) & 0xFFu);
+        ax[c] = __fadd_rn(ax[c], __fmul_rn(px, fa));
+        bx[c] = __fadd_rn(bx[c], __fmul_rn(px, fb));
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float p1 = __fmul_rn(ws.f, __fsub_rn(__fmul_rn(ax[c], ws.bsq), __fmul_rn(bx[c], ws.ab)));
+    const float p2 = __fmul_rn(ws.f, __fsub_rn(__fmul_rn(bx[c], ws.asq), __fmul_rn(ax[c], ws.ab)));
+    const uint32_t *s = c == 1 ? st.six : st.five;
+    r.snap[c] = s[quantize_endpoint(__fadd_rn(p1, 0.5f))];
+    r.snap[3 + c] = s[quantize_endpoint(__fadd_rn(p2, 0.5f))];
+  }
+}
+
+// err_diff of the refitted candidate (kInvalid where its endpoints would swap)
+// and its packed endpoints.
+__device__ __forceinline__ int refit_error(const PixBlock &t, const RefitValues &r, uint32_t cand, int orig_err,
+                                           uint32_t &eps) {
+  const uint32_t q1 = ((r.snap[0] << 8) & 0xF800u) | ((r.snap[1] << 3) & 0x07E0u) | ((r.snap[2] >> 3) & 0x1Fu);
+  const uint32_t q2 = ((r.snap[3] << 8) & 0xF800u) | ((r.snap[4] << 3) & 0x07E0u) | ((r.snap[5] >> 3) & 0x1Fu);
+  eps = q1 | (q2 << 16);
+  // the channel's four palette bytes: e1, e2, (2 e1 + e2) / 3, (e1 + 2 e2) / 3; x / 3
+  // is (x * 683) >> 11 for x <= 765, here shifted into its byte
+  uint32_t pal[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const uint32_t ends = __byte_perm(r.snap[c], r.snap[3 + c], 0x0040) & 0xFFFFu;
+    const uint32_t x2 = __dp4a(ends, 0x0102u, 0u), x3 = __dp4a(ends, 0x0201u, 0u);
+    pal[c] = ends | ((x2 * (683u << 5)) & 0x00FF0000u) | ((x3 * (683u << 13)) & 0xFF000000u);
+  }
+  uint32_t cross = 0, norm = 0;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const uint32_t sel = spread_nibbles((cand >> (8 * g)) & 0xFFu);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const uint32_t v = __byte_perm(pal[c], 0u, sel);
+      cross = __dp4a(t.pg[c][g], v, cross);
+      norm = __dp4a(v, v, norm);
+    }
+  }
+  const int sse = (int)t.sumsq - 2 * (int)cross + (int)norm;
+  return q1 > q2 ? (int)((uint32_t)sse / 48u) - orig_err : kInvalid;
+}
+
 }  // namespace mptc

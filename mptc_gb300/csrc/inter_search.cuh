@@ -204,186 +204,209 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) inter_dedup_kernel(Sea
 }
 
 // ------------------------------------------------------------ inter runs --
-// The same search for sa <= 8, one warp per run of RUN horizontally adjacent
-// blocks of a row. Their windows share all rows and overlap in all but
-// RUN - 1 columns, so the warp deduplicates the union of the windows (w2 rows
-// by w2 + RUN - 1 columns) once, recording for each distinct word the union
-// columns where it occurs (a bit mask); block k of the run then evaluates the
-// distinct words whose mask meets its columns k .. k + w2 - 1 and selects
-// over its own positions, exactly as the one-block search does.
+// The same search for sa <= 8, one warp per run of up to kRun horizontally
+// adjacent blocks of a row. Their windows share all rows and overlap in all but
+// a few columns, so the warp deduplicates the union of the windows (w2 rows of
+// at most w2 + kRun - 1 columns, a row at a time, lane = column) once, recording
+// for each distinct word the union columns where it occurs (a bit mask). The
+// pairs of a block and a distinct word of its window (other than its own) are
+// queued and evaluated 32 at a time across the blocks, so that the lanes stay
+// busy although a window holds some 33 words: refit_quick for each, refit_exact
+// for the few that it leaves out, queued until they fill a pass. Each result is
+// kept as a 16-bit rank per block and word. Per block the reference's selection
+// is then one minimum over the window's positions, the smallest rank at its
+// first position; only where a window holds an err_diff < 0 (12-19% of the
+// blocks) further passes find the first err_diff <= 0 and an err_diff < 0 in a
+// later row. The selected words of all blocks are refitted once more together
+// for their endpoints.
 // The hash table's empty marker is the first block's own word, which keeps a
-// dedicated slot 0 outside the table; out-of-frame positions carry the marker
-// and no column bit. The blocks of a run whose union holds more than
-// kRunWords distinct words (noisy content) are appended to a list that
+// dedicated slot 0 outside the table. The blocks of a run whose union holds more
+// than kRunWords distinct words (noisy content) are appended to a list that
 // inter_overflow_kernel searches afterwards with a CTA per block: those runs
 // cost several times a smooth one and, kept in one warp, would hold their SM
 // long after the other warps finished.
+// Bound by issue (84% of the slots), 927 warp instructions a block on the 1080p
+// test stream: evaluation 272 (73 of them the test for a near tie), deduplication
+// 194, lists 89, selection 67, the exact passes 130, the rest staging. 132 us a
+// frame, against 226 (1,566 instructions) with each block's words evaluated by
+// themselves from a table of float products in shared memory.
+constexpr int kRun = 8;
 constexpr int kRunWords = 128;  // distinct union words handled by the run table
 constexpr int kRunBuckets = 256;
+// err_diff e as a rank: 0 for e < 0, e + 1 for the others (err_diffs are at most
+// 65025), kNoRank where the refit would swap the endpoints
+constexpr uint32_t kNoRank = 0xFFFFu;
 
-template <int RUN>
 struct RunTab {
-  static constexpr int kCols = 16 + RUN - 1;  // union columns at sa = 8
-  static constexpr int kPos = 16 * kCols;     // union positions at sa = 8
-  static constexpr int kChunks = (kPos + 31) / 32;
-  // the marker, kRunWords words, and the up to 32 further new words of the
-  // chunk that crosses the limit
-  static constexpr int kSlots = 1 + kRunWords + 32;
-  uint32_t bkey[kRunBuckets];  // word, or the marker when empty
-  uint8_t bslot[kRunBuckets];
-  uint8_t pslot[kChunks * 32];  // slot of each union position
-  uint8_t list[kSlots];         // slots evaluated for the current block
-  uint16_t upos[kSlots];        // a union position holding the word
-  uint32_t key[kSlots];
-  uint32_t cols[kSlots];        // union columns holding the word (bit per column)
-  // the union's words while they are inserted, then each slot's err_diff
-  // (kSlots entries and the out-of-frame sentinel's kInvalid) and endpoint
-  // word (next kSlots) for the current block
+  static constexpr int kCols = 16 + kRun - 1;  // union columns at sa = 8
+  static constexpr int kStride = kCols + 1;
+  // the marker, kRunWords words, and the up to kCols further new words of the
+  // row that crosses the limit
+  static constexpr int kSlots = 1 + kRunWords + kCols;
   static constexpr int kSentinel = kSlots;  // slot of out-of-frame positions
-  static constexpr int kEval = 2 * kSlots + 1 > kChunks * 32 ? 2 * kSlots + 1 : kChunks * 32;
-  uint32_t ev[kEval];
-  __device__ __forceinline__ uint32_t *ucand() { return ev; }
-  __device__ __forceinline__ int *e() { return reinterpret_cast<int *>(ev); }
-  __device__ __forceinline__ uint32_t *eps() { return ev + kSlots + 1; }
+  PixBlock px[kRun];
+  int orig[kRun];
+  uint32_t own[kRun];
+  union {
+    struct {
+      uint32_t bkey[kRunBuckets];  // word, or the marker when empty
+      uint8_t bslot[kRunBuckets];
+    };
+    struct {  // pairs to evaluate: block << 8 | slot
+      uint16_t quick[32 + 32 * kRun], exact[64];
+    };
+  };
+  uint32_t key[kSlots];
+  uint32_t cols[kSlots];           // union columns holding the word (bit per column)
+  uint32_t at[kSlots];             // a block of the previous frame holding the word
+  uint8_t pslot[16 * kStride];     // slot of each union position
+  union {
+    uint32_t word[16][kCols];               // the union's words while they are inserted
+    uint16_t rank[kRun][kSlots + 1];  // of each block and word
+  };
 };
+
+// Evaluates a pair of a run from the integer sums; false where run_exact has to.
+__device__ __forceinline__ bool run_quick(const RunTab &rt, const float4 *wdesc, const SnapTables &st, uint32_t pair,
+                                          int &e) {
+  const int k = (int)(pair >> 8), s = (int)(pair & 255u);
+  const float4 d = __ldg(wdesc + rt.at[s]);
+  const WeightSums ws{d.x, d.y, d.z, d.w};
+  RefitValues r;
+  uint32_t eps;
+  const bool ok = refit_quick(rt.px[k], st, rt.key[s], ws, r);
+  e = refit_error(rt.px[k], r, rt.key[s], rt.orig[k], eps);
+  return ok;
+}
+// Evaluates a pair by the reference's own steps: its err_diff and endpoints.
+__device__ __forceinline__ uint2 run_exact(const RunTab &rt, const float4 *wdesc, const SnapTables &st, uint32_t pair) {
+  const int k = (int)(pair >> 8), s = (int)(pair & 255u);
+  const float4 d = __ldg(wdesc + rt.at[s]);
+  const WeightSums ws{d.x, d.y, d.z, d.w};
+  RefitValues r;
+  uint32_t eps;
+  refit_exact(rt.px[k], st, rt.key[s], ws, r);
+  const int e = refit_error(rt.px[k], r, rt.key[s], rt.orig[k], eps);
+  return make_uint2((uint32_t)e, eps);
+}
+__device__ __forceinline__ uint16_t run_rank(int e) {
+  return (uint16_t)(e == kInvalid ? kNoRank : (uint32_t)max(e, -1) + 1u);
+}
 
 // SA: the search area when fixed at compile time (its constants fold), 0 to
 // read it from P. A persistent grid: each warp takes the next unit of work
 // from *next_run (zero at launch), which keeps all warps busy to the end
-// although runs differ in cost. The units are the runs of the first
-// bh - tail_rows rows, then the blocks of the last tail_rows rows one by one
-// (runs of one block), so that the work left when the queue empties is short.
+// although runs differ in cost. run: blocks per run, at most RUN.
 template <int WARPS, int RUN, int SA>
 __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
-    inter_run_kernel(SearchParams P, uint32_t *next_run, int tail_rows, uint32_t *ovf_count, uint32_t *ovf_list) {
-  using Tab = RunTab<RUN>;
-  static_assert(Tab::kCols <= 32, "union columns must fit a 32-bit mask");
-  static_assert(sizeof(Tab) <= sizeof(DedupTab), "the one-block kernel's footprint: 32 warps per SM");
+    inter_run_kernel(SearchParams P, uint32_t *next_run, int run, uint32_t *ovf_count, uint32_t *ovf_list) {
+  using Tab = RunTab;
+  static_assert(RUN == kRun && 4 * kRun == 32, "a run's block rows take one lane each");
   static_assert(Tab::kSentinel <= 255 && Tab::kSlots - 1 <= kRunBuckets, "slots are bytes; buckets hold the words");
-  __shared__ BlockTab s_tab[WARPS];
   __shared__ Tab s_run[WARPS];
-  __shared__ uint8_t s_snap5[256], s_snap6[256];
-  build_snap_tables(s_snap5, s_snap6);
+  __shared__ SnapTables s_snap;
+  build_snap_edges(s_snap);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  BlockTab &tab = s_tab[warp];
   Tab &rt = s_run[warp];
   const unsigned lt_mask = (1u << lane) - 1u;
   const int sa = SA ? SA : P.sa;
-  const int w2 = 2 * sa, ucols = w2 + RUN - 1, upos = w2 * ucols;
-  // the lane's first union position (row, column) and the step to its next
-  const int urow0 = lane / ucols, ucol0 = lane - urow0 * ucols;
-  const int drow = 32 / ucols, dcol = 32 - drow * ucols;
-  // pos / w2 and u / ucols as multiplies-high: exact below 2^16 for divisors <= 126
-  const uint32_t w2_magic = 0xFFFFFFFFu / (uint32_t)w2 + 1u, uc_magic = 0xFFFFFFFFu / (uint32_t)ucols + 1u;
-  const uint32_t wmask = (1u << w2) - 1u;
-  // the lane's first window position (row, column) and the step to its next
-  const int npos = w2 * w2, prow0 = lane / w2, pcol0 = lane - prow0 * w2;
-  const int pdrow = 32 / w2, pdcol = 32 - pdrow * w2;
+  const int w2 = 2 * sa;
   const uint32_t *prev_hi = reinterpret_cast<const uint32_t *>(P.prev) + 1;
-  const int runs_per_row = (P.bw + RUN - 1) / RUN, main_rows = P.bh - tail_rows;
-  const int nmain = runs_per_row * main_rows, nunits = nmain + tail_rows * P.bw;
   for (;;) {
     int unit = 0;
     if (lane == 0) unit = (int)atomicAdd(next_run, 1u);
     unit = __shfl_sync(kFull, unit, 0);
-    if (unit >= nunits) break;
-    int by, bx0, nb;
-    if (unit < nmain) {
-      by = unit / runs_per_row;
-      bx0 = (unit - by * runs_per_row) * RUN;
-      nb = min(RUN, P.bw - bx0);
-    } else {
-      const int b = main_rows * P.bw + (unit - nmain);
-      by = b / P.bw;
-      bx0 = b - by * P.bw;
-      nb = 1;
-    }
-    const int j0 = by - sa, i0 = bx0 - sa, ucols_used = w2 + nb - 1;
+    const int per_row = (P.bw + run - 1) / run, by = unit / per_row;
+    if (by >= P.bh) break;
+    const int bx0 = (unit - by * per_row) * run, nb = min(run, P.bw - bx0);
+    const int j0 = by - sa, i0 = bx0 - sa;
     const uint32_t marker = (uint32_t)(P.stb[by * P.bw + bx0] >> 32);
-    for (int b = lane; b < kRunBuckets; b += 32) rt.bkey[b] = marker;
-    if (lane == 0) {
-      rt.key[0] = marker;
-      rt.cols[0] = 0;
+    for (int b = lane; b < kRunBuckets / 4; b += 32)
+      reinterpret_cast<uint4 *>(rt.bkey)[b] = make_uint4(marker, marker, marker, marker);
+    if (lane < nb) {
+      rt.orig[lane] = P.orig_err[by * P.bw + bx0 + lane];
+      rt.own[lane] = (uint32_t)(P.stb[by * P.bw + bx0 + lane] >> 32);
+    }
+    // the union's words, all loads first so their latencies overlap
+    const bool col_in = lane < w2 + nb - 1 && i0 + lane >= 0 && i0 + lane < P.bw;
+    const unsigned colm = __ballot_sync(kFull, col_in);
+    if (lane < Tab::kCols) {
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+        if (r < w2) {
+          const int j = j0 + r;
+          rt.word[r][lane] = col_in && j >= 0 && j < P.bh ? __ldg(prev_hi + 2 * (size_t)(j * P.bw + i0 + lane)) : marker;
+        }
     }
     __syncwarp();
-    // the union's words, all loads first so their latencies overlap
-    uint32_t *ucand = rt.ucand();
-    unsigned valid = 0;
+    // the blocks' pixels, one block row per lane
     {
-      int urow = urow0, ucol = ucol0;
+      const int k = lane >> 2, r = lane & 3;
+      uint32_t c0 = 0, c1 = 0, c2 = 0;
+      if (k < nb) load_channels(P.rgb, P.width, bx0 + k, 4 * by + r, c0, c1, c2);
+      uint32_t s0 = __dp4a(c0, 0x01010101u, 0u), s1 = __dp4a(c1, 0x01010101u, 0u), s2 = __dp4a(c2, 0x01010101u, 0u);
+      uint32_t sq = __dp4a(c0, c0, __dp4a(c1, c1, __dp4a(c2, c2, 0u)));
 #pragma unroll
-      for (int c = 0; c < Tab::kChunks; ++c) {
-        const int j = j0 + urow, i = i0 + ucol;
-        uint32_t cand = marker;
-        if (32 * c + lane < upos && ucol < ucols_used && i >= 0 && j >= 0 && i < P.bw && j < P.bh) {
-          cand = __ldg(prev_hi + 2 * (size_t)(j * P.bw + i));
-          valid |= 1u << c;
-        }
-        ucand[32 * c + lane] = cand;
-        urow += drow;
-        ucol += dcol;
-        if (ucol >= ucols) {
-          ucol -= ucols;
-          ++urow;
-        }
+      for (int o = 1; o <= 2; o <<= 1) {
+        s0 += __shfl_xor_sync(kFull, s0, o);
+        s1 += __shfl_xor_sync(kFull, s1, o);
+        s2 += __shfl_xor_sync(kFull, s2, o);
+        sq += __shfl_xor_sync(kFull, sq, o);
+      }
+      if (k < nb) {
+        PixBlock &px = rt.px[k];
+        px.pg[0][r] = c0;
+        px.pg[1][r] = c1;
+        px.pg[2][r] = c2;
+        if (r == 0) *reinterpret_cast<uint4 *>(px.sum) = make_uint4(s0, s1, s2, sq);
       }
     }
-    __syncwarp();
+    // the distinct words, row by row: a word's first lane looks it up
     int nuniq = 1;
+    uint32_t mark_cols = 0, mark_at = 0;  // the marker's
     bool overflow = false;
-    {
-      int ucol = ucol0;
 #pragma unroll 1
-      for (int c = 0; c < Tab::kChunks; ++c) {
-        const uint32_t cand = ucand[32 * c + lane];
-        const bool ok = (valid >> c) & 1u;
-        const unsigned peers = __match_any_sync(kFull, cand);
-        const int leader = __ffs(peers) - 1;
-        const uint32_t colbits = __reduce_or_sync(peers, ok ? 1u << ucol : 0u);
-        const unsigned okm = __ballot_sync(kFull, ok);
-        uint32_t b = 0;
-        int slot = 0;
+    for (int r = 0; r < w2; ++r) {
+      const int j = j0 + r;
+      int slot = Tab::kSentinel;
+      if (j >= 0 && j < P.bh) {  // warp-uniform
+        const uint32_t cand = lane < Tab::kCols ? rt.word[r][lane] : marker;
+        const unsigned peers = __match_any_sync(kFull, cand) & colm;
         bool is_new = false;
-        if (lane == leader && colbits) {  // groups of out-of-frame positions only are skipped
-          if (cand == marker) {
-            if (rt.cols[0] == 0) rt.upos[0] = (uint16_t)(32 * c + __ffs(peers & okm) - 1);
-            rt.cols[0] |= colbits;
-          } else {
-            b = dedup_hash(cand);
-            for (int probe = 0; probe < kRunBuckets; ++probe) {
-              const uint32_t old = atomicCAS(&rt.bkey[b], marker, cand);
-              if (old == marker) {
-                is_new = true;
-                break;
-              }
-              if (old == cand) {
-                slot = rt.bslot[b];  // inserted by an earlier chunk
-                rt.cols[slot] |= colbits;
-                break;
-              }
-              b = (b + 1) & (kRunBuckets - 1);
-            }
+        uint32_t b = 0;
+        slot = 0;
+        if (cand == marker) {
+          mark_cols |= peers;
+          if (peers) mark_at = (uint32_t)(j * P.bw + i0 + __ffs(peers) - 1);
+        } else if (lane == __ffs(peers) - 1) {
+          b = dedup_hash(cand);
+          uint32_t old;
+          while ((old = atomicCAS(&rt.bkey[b], marker, cand)) != marker && old != cand)
+            b = (b + 1) & (kRunBuckets - 1);  // ends: at most kSlots - 1 words in kRunBuckets
+          is_new = old == marker;
+          if (!is_new) {  // inserted by an earlier row
+            slot = rt.bslot[b];
+            rt.cols[slot] |= peers;
           }
         }
         const unsigned newm = __ballot_sync(kFull, is_new);
-        if (is_new) {  // the leader's own position holds the word
+        if (is_new) {
           slot = nuniq + __popc(newm & lt_mask);
           rt.bslot[b] = (uint8_t)slot;
           rt.key[slot] = cand;
-          rt.cols[slot] = colbits;
-          rt.upos[slot] = (uint16_t)(32 * c + lane);
+          rt.cols[slot] = peers;
+          rt.at[slot] = (uint32_t)(j * P.bw + i0 + lane);
         }
-        slot = __shfl_sync(kFull, slot, leader);
-        rt.pslot[32 * c + lane] = (uint8_t)(ok ? slot : Tab::kSentinel);
+        slot = __shfl_sync(kFull, slot, max(__ffs(peers) - 1, 0));
+        if (!col_in) slot = Tab::kSentinel;
         nuniq += __popc(newm);
-        __syncwarp();  // this chunk's slot writes land before later chunks read them
-        if (nuniq > 1 + kRunWords) {  // warp-uniform
-          overflow = true;
-          break;
-        }
-        ucol += dcol;
-        if (ucol >= ucols) ucol -= ucols;
+        __syncwarp();  // this row's slot writes land before later rows read them
+      }
+      if (lane < Tab::kCols) rt.pslot[r * Tab::kStride + lane] = (uint8_t)slot;
+      if (nuniq > 1 + kRunWords) {  // warp-uniform
+        overflow = true;
+        break;
       }
     }
     if (overflow) {
@@ -391,77 +414,148 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
         const uint32_t at = atomicAdd(ovf_count, (uint32_t)nb);
         for (int k = 0; k < nb; ++k) ovf_list[at + k] = (uint32_t)(by * P.bw + bx0 + k);
       }
+      __syncwarp();
       continue;
     }
-    if (lane == 0) rt.e()[Tab::kSentinel] = kInvalid;
-    for (int k = 0; k < nb; ++k) {
-      const int bx = bx0 + k, idx = by * P.bw + bx;
-      const uint64_t stb = P.stb[idx];
-      const uint32_t own = (uint32_t)(stb >> 32);
-      const int orig = P.orig_err[idx];
-      const int sumsq = stage_block(tab, P.rgb, P.width, bx, by, lane);
-      const PixelGroups pg = load_groups(tab);
-      // the distinct words of this block's window; its own word needs no refit
-      const uint32_t win = wmask << k;
-      int nl = 0;
-      for (int s0 = 0; s0 < nuniq; s0 += 32) {
-        const int s = s0 + lane;
-        bool take = false;
-        if (s < nuniq && (rt.cols[s] & win)) {
-          if (rt.key[s] == own)
-            rt.e()[s] = 0;
-          else
-            take = true;
-        }
-        const unsigned tm = __ballot_sync(kFull, take);
-        if (take) rt.list[nl + __popc(tm & lt_mask)] = (uint8_t)s;
-        nl += __popc(tm);
-      }
-      __syncwarp();
-      for (int q = lane; q < nl; q += 32) {
-        const int s = rt.list[q];
-        const int u = rt.upos[s];
-        const int ur = (int)__umulhi((uint32_t)u, uc_magic);
-        const float4 d = __ldg(P.wdesc + (size_t)((j0 + ur) * P.bw + i0 + u - ur * ucols));
-        const WeightSums ws{d.x, d.y, d.z, d.w};
-        uint32_t eps = 0;
-        int refit = 0;
-        rt.e()[s] = eval_candidate(tab, pg, s_snap5, s_snap6, rt.key[s], ws, own, orig, sumsq, eps, refit);
-        rt.eps()[s] = eps;
-      }
-      __syncwarp();
-      // the block's positions in scan order, 32 at a time
-      LaneSel sel;
-      {
-        int row = prow0, col = pcol0;
-#pragma unroll 1
-        for (int pos = lane; pos < npos; pos += 32) {
-          sel.add(pos, row, rt.e()[rt.pslot[row * ucols + col + k]]);
-          row += pdrow;
-          col += pdcol;
-          if (col >= w2) {
-            col -= w2;
-            ++row;
-          }
-        }
-      }
-      int m;
-      const int sp = warp_select(sel, w2, m);
+    {  // the marker's lanes (a word's peers are the same row by row, its lanes are not)
+      const uint32_t c = __reduce_or_sync(kFull, mark_cols), at = __reduce_max_sync(kFull, mark_at);
       if (lane == 0) {
-        uint64_t word = 0;
-        if (sp >= 0 && m <= P.thr) {
-          const int row = (int)__umulhi((uint32_t)sp, w2_magic), col = sp - row * w2;
-          const int slot = rt.pslot[row * ucols + col + k];
-          const uint32_t cand = rt.key[slot];
-          const uint64_t blk = cand == own ? stb : ((uint64_t)rt.eps()[slot] | ((uint64_t)cand << 32));
-          P.final_blk[idx] = blk;
-          P.motion[idx] = (uint16_t)((col | 0x80) | ((row | 0x80) << 8));
-          word = done_word(blk);
-        }
-        P.done[idx] = word;
+        rt.key[0] = marker;
+        rt.cols[0] = c;
+        rt.at[0] = at;
       }
-      __syncwarp();
     }
+    __syncwarp();
+    // the pairs, queued and evaluated
+    int nquick = 0, nexact = 0;
+#pragma unroll 1
+    for (int s0 = 0; s0 < nuniq; s0 += 32) {
+      const int s = s0 + lane;
+      // the blocks whose window holds the word: bit k, columns k .. k + w2 - 1
+      uint32_t take = 0;
+      if (s < nuniq) {
+        take = rt.cols[s];
+        if (SA == 8) {
+          take |= take >> 1;
+          take |= take >> 2;
+          take |= take >> 4;
+          take |= take >> 8;
+        } else {
+          const uint32_t c = take;
+          for (int i = 1; i < w2; ++i) take |= c >> i;
+        }
+        take &= (1u << nb) - 1u;
+        const uint32_t key = rt.key[s];
+        uint32_t own = 0;
+#pragma unroll
+        for (int k = 0; k < kRun; ++k) own |= key == rt.own[k] ? 1u << k : 0u;
+        for (own &= take; own; own &= own - 1u) {  // the block's own word: err_diff 0, no refit
+          const int k = __ffs(own) - 1;
+          rt.rank[k][s] = 1u;
+          take &= ~(1u << k);
+        }
+      }
+      int at = __popc(take);
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(kFull, at, d);
+        if (lane >= d) at += v;
+      }
+      const int total = __shfl_sync(kFull, at, 31);
+      at += nquick - __popc(take);
+#pragma unroll
+      for (int k = 0; k < kRun; ++k)
+        if ((take >> k) & 1u) rt.quick[at++] = (uint16_t)((k << 8) | s);
+      nquick += total;
+      __syncwarp();
+      const bool last = s0 + 32 >= nuniq;
+      while (nquick >= 32 || (last && nquick + nexact > 0)) {
+        // full passes from the queues' ends; what is left with the last words
+        if (nquick >= 32 || (last && nquick > 0)) {
+          const int n = min(nquick, 32);
+          nquick -= n;
+          bool out = false;
+          uint32_t pair = 0;
+          if (lane < n) {
+            pair = rt.quick[nquick + lane];
+            int e;
+            out = !run_quick(rt, P.wdesc, s_snap, pair, e);
+            rt.rank[pair >> 8][pair & 255u] = run_rank(e);
+          }
+          const unsigned om = __ballot_sync(kFull, out);
+          if (out) rt.exact[nexact + __popc(om & lt_mask)] = (uint16_t)pair;
+          nexact += __popc(om);
+          __syncwarp();
+        }
+        if (nexact >= 32 || (last && nquick == 0 && nexact > 0)) {
+          const int n = min(nexact, 32);
+          nexact -= n;
+          if (lane < n) {
+            const uint32_t pair = rt.exact[nexact + lane];
+            rt.rank[pair >> 8][pair & 255u] = run_rank((int)run_exact(rt, P.wdesc, s_snap, pair).x);
+          }
+          __syncwarp();
+        }
+      }
+    }
+    if (lane < nb) rt.rank[lane][Tab::kSentinel] = (uint16_t)kNoRank;
+    __syncwarp();
+    // lane k: its block's selected position + 1 (0: none) << 8 | slot
+    uint32_t win = 0;
+#pragma unroll 1
+    for (int k = 0; k < nb; ++k) {
+      const uint16_t *rank = rt.rank[k];
+      const uint8_t *pslot = rt.pslot + k;
+      // rank << 8 | position, in scan order (rows, then columns)
+      uint32_t best = 0xFFFFFFFFu;
+      auto each = [&](auto f) {
+        if (SA == 8) {
+          const uint8_t *at = pslot + (lane >> 4) * Tab::kStride + (lane & 15);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) f(rank[at[2 * c * Tab::kStride]], (uint32_t)(32 * c + lane));
+        } else {
+#pragma unroll 1
+          for (int p = lane; p < w2 * w2; p += 32) f(rank[pslot[p / w2 * Tab::kStride + p % w2]], (uint32_t)p);
+        }
+      };
+      each([&](uint32_t v, uint32_t p) { best = min(best, (v << 8) | p); });
+      best = __reduce_min_sync(kFull, best);
+      int pos = -1;
+      if (best < 256u) {  // an err_diff < 0
+        if (P.thr >= 0) {
+          uint32_t first = 256u;
+          int last = -1;
+          each([&](uint32_t v, uint32_t p) {
+            if (v <= 1u) first = min(first, p);
+            if (v == 0u) last = max(last, (int)((p / (uint32_t)w2 << 8) | (255u - p)));
+          });
+          first = __reduce_min_sync(kFull, first);
+          last = __reduce_max_sync(kFull, last);
+          pos = (last >> 8) > (int)(first / (uint32_t)w2) ? 255 - (last & 255) : (int)first;
+        }
+      } else if (best < kNoRank << 8 && (int)(best >> 8) - 1 <= P.thr) {
+        pos = (int)(best & 255u);
+      }
+      if (lane == k && pos >= 0)
+        win = ((uint32_t)pos + 1u) << 8 | pslot[pos / w2 * Tab::kStride + pos % w2];
+    }
+    if (lane < nb) {
+      const int idx = by * P.bw + bx0 + lane;
+      uint64_t word = 0;
+      if (win != 0u) {
+        const uint32_t s = win & 255u, pos = (win >> 8) - 1u;
+        uint64_t blk = P.stb[idx];
+        if (rt.key[s] != rt.own[lane]) {
+          blk = (uint64_t)run_exact(rt, P.wdesc, s_snap, (uint32_t)lane << 8 | s).y | ((uint64_t)rt.key[s] << 32);
+        }
+        const uint32_t row = pos / (uint32_t)w2, col = pos - row * (uint32_t)w2;
+        P.final_blk[idx] = blk;
+        P.motion[idx] = (uint16_t)((col | 0x80) | ((row | 0x80) << 8));
+        word = done_word(blk);
+      }
+      P.done[idx] = word;
+    }
+    __syncwarp();
   }
 }
 

@@ -22,7 +22,7 @@
 namespace {
 
 constexpr int kSearchWarps = 4;     // inter search: warps per CTA
-constexpr int kInterRun = 8;        // inter search at sa <= 8: blocks per warp (a run of a row)
+constexpr int kInterRun = mptc::kRun;  // inter search at sa <= 8: blocks per warp (a run of a row)
 constexpr int kIntraThreads = 256;  // intra search: one block per CTA
 constexpr int kSweeps = 6;          // default fixed-point sweeps of an inter frame's intra pass
 constexpr int kMaxSweeps = 32;
@@ -369,20 +369,24 @@ int launch_inter_search(const mptc::SearchParams &P, int warps, uint32_t *work, 
       mptc::inter_dedup_kernel<4><<<(nblk + 3) / 4, 4 * 32, 0, s>>>(P);
     return 1;
   }
-  const int nruns = (P.bw + kInterRun - 1) / kInterRun * P.bh;
-  const int ctas = std::min((nruns + warps - 1) / warps, sm_count * (32 / warps));
-  // the last rows one block at a time: about two blocks per warp
-  const int tail = std::min(P.bh, (2 * ctas * warps + P.bw - 1) / P.bw);
+  // runs of kInterRun blocks, in a small frame short enough to give every warp
+  // one (256x256, runs of one block: 110 us an inter frame against 122 with runs
+  // of 8). A shorter run costs more per block (the union's words are looked up
+  // once per run): ending a 1080p frame with runs of 4 or 2 blocks for an even
+  // finish took 249 and 253 us against 245.
+  const int slots = sm_count * 32, run = std::min(kInterRun, (nblk + slots - 1) / slots);
+  const int units = (P.bw + run - 1) / run * P.bh;
+  const int ctas = std::min((units + warps - 1) / warps, slots / warps);
   uint32_t *next = work + 7, *novf = work + 8;
   // the default search area 8 with its window constants folded
   if (P.sa == 8 && warps == 2)
-    mptc::inter_run_kernel<2, kInterRun, 8><<<ctas, 2 * 32, 0, s>>>(P, next, tail, novf, ovf_list);
+    mptc::inter_run_kernel<2, mptc::kRun, 8><<<ctas, 2 * 32, 0, s>>>(P, next, run, novf, ovf_list);
   else if (P.sa == 8)
-    mptc::inter_run_kernel<4, kInterRun, 8><<<ctas, 4 * 32, 0, s>>>(P, next, tail, novf, ovf_list);
+    mptc::inter_run_kernel<4, mptc::kRun, 8><<<ctas, 4 * 32, 0, s>>>(P, next, run, novf, ovf_list);
   else if (warps == 2)
-    mptc::inter_run_kernel<2, kInterRun, 0><<<ctas, 2 * 32, 0, s>>>(P, next, tail, novf, ovf_list);
+    mptc::inter_run_kernel<2, mptc::kRun, 0><<<ctas, 2 * 32, 0, s>>>(P, next, run, novf, ovf_list);
   else
-    mptc::inter_run_kernel<4, kInterRun, 0><<<ctas, 4 * 32, 0, s>>>(P, next, tail, novf, ovf_list);
+    mptc::inter_run_kernel<4, mptc::kRun, 0><<<ctas, 4 * 32, 0, s>>>(P, next, run, novf, ovf_list);
   // the overflow list is short: four CTAs per SM, idle ones return at once
   mptc::inter_overflow_kernel<256><<<std::min(4 * sm_count, nblk), 256, 0, s>>>(P, ovf_list, novf);
   return 2;
