@@ -7,6 +7,17 @@
 
 namespace mptc {
 
+// Programmatic dependent launch: the CTAs of a kernel launched that way start while
+// the kernel before it in the stream still runs. Every such kernel calls depend() in
+// all its threads before it touches global memory: it waits until the kernel before
+// has completed with its writes visible, which itself has waited for the one before
+// it, so the order is the stream's. A short kernel then lets the next one's CTAs
+// start (release_next()) where SMs have room; a long one does not, whose successor's
+// waiting CTAs would keep other streams' kernels off the SMs, and releases it as its
+// CTAs exit.
+__device__ __forceinline__ void depend() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

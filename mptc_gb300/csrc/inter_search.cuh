@@ -189,6 +189,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) inter_dedup_kernel(Sea
   __shared__ uint8_t s_snap5[256], s_snap6[256];
   build_snap_tables(s_snap5, s_snap6);
   __syncthreads();
+  depend();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   BlockTab &tab = s_tab[warp];
   const int nblk = P.bw * P.bh;
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
   __shared__ SnapTables s_snap;
   build_snap_edges(s_snap);
   __syncthreads();
+  depend();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   Tab &rt = s_run[warp];
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -560,13 +562,21 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
 }
 
 // Weight sums of the refit for every block's index word (the candidates the
-// next inter search reads), one thread per block.
+// next search reads), one thread per block. As the first kernel of a search it
+// also zeroes the frame's work words and, for an intra frame, the completion
+// words (zeroed: n of them, or null), instead of a memset each before it.
 __global__ void __launch_bounds__(256) weight_desc_kernel(const uint64_t *__restrict__ blocks, int n,
-                                                          float4 *__restrict__ desc) {
+                                                          float4 *__restrict__ desc, uint32_t *__restrict__ work,
+                                                          int n_work, uint64_t *__restrict__ zeroed) {
   __shared__ float4 s_wk[4];
   build_weight_table(s_wk);
   __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  depend();
+  release_next();
+  const int first = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int i = first; i < n_work; i += gridDim.x * blockDim.x) work[i] = 0u;
+  for (int i = first; i < n; i += gridDim.x * blockDim.x) {
+    if (zeroed) zeroed[i] = 0ull;
     const WeightSums w = weight_sums((uint32_t)(__ldg(blocks + i) >> 32), s_wk);
     desc[i] = make_float4(w.asq, w.bsq, w.ab, w.f);
   }
@@ -634,6 +644,8 @@ template <int THREADS>
 __global__ void __launch_bounds__(THREADS) inter_overflow_kernel(SearchParams P, const uint32_t *__restrict__ list,
                                                                  const uint32_t *__restrict__ count) {
   static_assert(THREADS >= 256, "one thread per position of a 16x16 window");
+  depend();
+  release_next();
   const int n = (int)__ldcg(count);
   if ((int)blockIdx.x >= n) return;  // the whole CTA, before its barriers
   __shared__ BlockTab s_tab;

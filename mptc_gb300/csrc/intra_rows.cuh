@@ -554,6 +554,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) intra_rows_kernel(SearchParams
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = cluster_rank(), ncta = cluster_size();
   build_snap_tables(S.snap5, S.snap6);
+  depend();
   const int sa = P.sa, bw = P.bw, groups = (bw + kRowGroup - 1) / kRowGroup;
   const uint32_t next_hist = cluster_map(S.hist, (rank + 1u) % ncta);
   for (;;) {

@@ -165,7 +165,8 @@ __global__ void __launch_bounds__(THREADS, 4) intra_search_kernel(SearchParams P
                                                                const uint32_t *__restrict__ n_pending_dev,
                                                                int n_pending_host,
                                                                const uint32_t *__restrict__ run_flag = nullptr) {
-  if (run_flag && __ldcg(run_flag) == 0u) return;  // the sweeps below converged
+  depend();
+  if (run_flag && __ldcg(run_flag) == 0u) return;  // the sweeps before converged
   __shared__ BlockTab s_tab;
   __shared__ EvalCache s_cache;
   __shared__ uint8_t s_snap5[256], s_snap6[256];
@@ -250,7 +251,6 @@ __global__ void __launch_bounds__(THREADS, 3) intra_sweep_kernel(SearchParams P,
                                                               uint32_t *__restrict__ changed_out,
                                                               SweepPartial *__restrict__ part, int part_cap,
                                                               bool first) {
-  if (__ldcg(changed_in) == 0u) return;
   __shared__ BlockTab s_tab;
   __shared__ EvalCache s_cache;
   __shared__ uint8_t s_snap5[256], s_snap6[256];
@@ -259,6 +259,9 @@ __global__ void __launch_bounds__(THREADS, 3) intra_sweep_kernel(SearchParams P,
   __shared__ int s_sumsq;
   build_snap_tables(s_snap5, s_snap6);
   build_weight_table(s_wk);
+  depend();
+  release_next();
+  if (__ldcg(changed_in) == 0u) return;
   CtaReduce<THREADS> red{s_red, 0};
   CacheUse cache;
   const int tid = threadIdx.x, lane = tid & 31;

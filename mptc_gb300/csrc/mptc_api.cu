@@ -291,6 +291,25 @@ __global__ void alu_probe_kernel(int iters, int32_t *sink) {
 
 namespace {
 
+// Launches a kernel that calls depend() behind the kernel before it in the stream
+// (programmatic dependent launch). Used inside a frame's chain of kernels, not
+// behind an event wait. A frame is a chain of some 13 kernels of 3 to 20 us; launched
+// this way, with the work area zeroed by the first of them instead of two memsets, an
+// inter frame takes 212 us at 1080p (245 before) and 74.5 us at 256x256 (107).
+template <typename... Par, typename... Arg>
+void launch_chain(void (*kernel)(Par...), int grid, int threads, cudaStream_t s, Arg... arg) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, Par(arg)...);
+}
+
 // The intra pass of an inter frame: fixed-point sweeps over the open blocks,
 // then the exact dataflow kernel only if the sweeps did not converge.
 // Sweeps to run for a configuration's intra_sweeps value.
@@ -305,46 +324,66 @@ int launch_intra_sweeps(const mptc::SearchParams &P, const uint32_t *pending, co
                         uint32_t *sweep, int n, int grid, int sweeps, mptc::SweepPartial *part, int part_cap,
                         cudaStream_t s) {
   if (sweeps == 0) {
-    mptc::intra_search_kernel<kIntraThreads><<<grid, kIntraThreads, 0, s>>>(P, pending, n_pending, -1);
+    launch_chain(mptc::intra_search_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, -1, nullptr);
     return 1;
   }
   // three estimate buffers: sweep k reads E[k % 3] and, for its skip test,
   // E[(k + 2) % 3] (the estimates sweep k-1 read), and writes E[(k + 1) % 3]
   uint32_t *est[3] = {sweep, sweep + n, sweep + 2 * (size_t)n}, *changed = sweep + 3 * (size_t)n;
   for (int k = 0; k < sweeps; ++k)
-    mptc::intra_sweep_kernel<kIntraThreads><<<grid, kIntraThreads, 0, s>>>(
-        P, pending, n_pending, est[k % 3], est[(k + 2) % 3], est[(k + 1) % 3], changed + k, changed + k + 1, part,
-        part_cap, k == 0);
-  mptc::intra_search_kernel<kIntraThreads><<<grid, kIntraThreads, 0, s>>>(P, pending, n_pending, -1,
-                                                                          changed + sweeps);
+    launch_chain(mptc::intra_sweep_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, est[k % 3],
+                 est[(k + 2) % 3], est[(k + 1) % 3], changed + k, changed + k + 1, part, part_cap, k == 0);
+  launch_chain(mptc::intra_search_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, -1,
+               changed + sweeps);
   return sweeps + 1;
 }
 
-// The intra search of a whole intra frame (P.done zeroed): the row pipeline on
-// `ctas` SMs at sa <= 8 (after the weight sums of the stb words it reads), the
-// block dataflow on `grid` CTAs for larger windows. Returns the number of
-// kernels launched.
-int launch_intra_frame(const mptc::SearchParams &P, float4 *wdesc, const uint32_t *order, int grid, int ctas,
-                       cudaStream_t s) {
+// First kernel of a search: the weight sums of the words it reads (the previous
+// frame's, or an intra frame's own stb words), the frame's work words zeroed and,
+// for an intra frame, its completion words. An intra frame with a larger window
+// needs no weight sums. chained: the kernel before it in the stream is this frame's
+// stb encode. Returns the number of kernels launched.
+int launch_begin(const mptc::SearchParams &P, float4 *wdesc, int ntiles, bool chained, cudaStream_t s) {
+  const int nblk = P.bw * P.bh;
+  if (!P.prev && P.sa > 8) {
+    cudaMemsetAsync(P.work, 0, work_bytes(ntiles), s);
+    cudaMemsetAsync(P.done, 0, (size_t)nblk * sizeof(uint64_t), s);
+    return 0;
+  }
+  const int grid = (nblk + 255) / 256, n_work = (int)(work_bytes(ntiles) / sizeof(uint32_t));
+  const uint64_t *words = P.prev ? P.prev : P.stb;
+  uint64_t *zeroed = P.prev ? nullptr : P.done;
+  if (chained)
+    launch_chain(mptc::weight_desc_kernel, grid, 256, s, words, nblk, wdesc, P.work, n_work, zeroed);
+  else
+    mptc::weight_desc_kernel<<<grid, 256, 0, s>>>(words, nblk, wdesc, P.work, n_work, zeroed);
+  return 1;
+}
+
+// The intra search of a whole intra frame, behind launch_begin: the row pipeline
+// on `ctas` SMs at sa <= 8, the block dataflow on `grid` CTAs for larger windows.
+// Returns the number of kernels launched.
+int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int grid, int ctas, cudaStream_t s) {
   const int nblk = P.bw * P.bh;
   if (P.sa > 8) {
     mptc::intra_search_kernel<kIntraThreads><<<grid, kIntraThreads, 0, s>>>(P, order, nullptr, nblk);
     return 1;
   }
-  mptc::weight_desc_kernel<<<(nblk + 255) / 256, 256, 0, s>>>(P.stb, nblk, wdesc);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(mptc::kRowCluster * std::max(1, std::min(P.bh, ctas / mptc::kRowCluster)));
   cfg.blockDim = dim3(mptc::kRowThreads);
   cfg.dynamicSmemBytes = sizeof(mptc::RowShared);
   cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = mptc::kRowCluster;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2]{};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = mptc::kRowCluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
   cudaLaunchKernelEx(&cfg, mptc::intra_rows_kernel, P);
-  return 2;
+  return 1;
 }
 
 // The row pipeline's shared memory (its warps' tables).
@@ -364,31 +403,31 @@ int launch_inter_search(const mptc::SearchParams &P, int warps, uint32_t *work, 
   const int nblk = P.bw * P.bh;
   if (P.sa > 8) {
     if (warps == 2)
-      mptc::inter_dedup_kernel<2><<<(nblk + 1) / 2, 2 * 32, 0, s>>>(P);
+      launch_chain(mptc::inter_dedup_kernel<2>, (nblk + 1) / 2, 2 * 32, s, P);
     else
-      mptc::inter_dedup_kernel<4><<<(nblk + 3) / 4, 4 * 32, 0, s>>>(P);
+      launch_chain(mptc::inter_dedup_kernel<4>, (nblk + 3) / 4, 4 * 32, s, P);
     return 1;
   }
   // runs of kInterRun blocks, in a small frame short enough to give every warp
   // one (256x256, runs of one block: 110 us an inter frame against 122 with runs
   // of 8). A shorter run costs more per block (the union's words are looked up
   // once per run): ending a 1080p frame with runs of 4 or 2 blocks for an even
-  // finish took 249 and 253 us against 245.
+  // finish took 249 and 253 us against 245 (before launch_chain).
   const int slots = sm_count * 32, run = std::min(kInterRun, (nblk + slots - 1) / slots);
   const int units = (P.bw + run - 1) / run * P.bh;
   const int ctas = std::min((units + warps - 1) / warps, slots / warps);
   uint32_t *next = work + 7, *novf = work + 8;
   // the default search area 8 with its window constants folded
   if (P.sa == 8 && warps == 2)
-    mptc::inter_run_kernel<2, mptc::kRun, 8><<<ctas, 2 * 32, 0, s>>>(P, next, run, novf, ovf_list);
+    launch_chain(mptc::inter_run_kernel<2, mptc::kRun, 8>, ctas, 2 * 32, s, P, next, run, novf, ovf_list);
   else if (P.sa == 8)
-    mptc::inter_run_kernel<4, mptc::kRun, 8><<<ctas, 4 * 32, 0, s>>>(P, next, run, novf, ovf_list);
+    launch_chain(mptc::inter_run_kernel<4, mptc::kRun, 8>, ctas, 4 * 32, s, P, next, run, novf, ovf_list);
   else if (warps == 2)
-    mptc::inter_run_kernel<2, mptc::kRun, 0><<<ctas, 2 * 32, 0, s>>>(P, next, run, novf, ovf_list);
+    launch_chain(mptc::inter_run_kernel<2, mptc::kRun, 0>, ctas, 2 * 32, s, P, next, run, novf, ovf_list);
   else
-    mptc::inter_run_kernel<4, mptc::kRun, 0><<<ctas, 4 * 32, 0, s>>>(P, next, run, novf, ovf_list);
+    launch_chain(mptc::inter_run_kernel<4, mptc::kRun, 0>, ctas, 4 * 32, s, P, next, run, novf, ovf_list);
   // the overflow list is short: four CTAs per SM, idle ones return at once
-  mptc::inter_overflow_kernel<256><<<std::min(4 * sm_count, nblk), 256, 0, s>>>(P, ovf_list, novf);
+  launch_chain(mptc::inter_overflow_kernel<256>, std::min(4 * sm_count, nblk), 256, s, P, ovf_list, novf);
   return 2;
 }
 
@@ -604,17 +643,10 @@ mptc_status reencode_check(mptc_ctx *ctx, const uint8_t *rgb_dev, const uint64_t
   return MPTC_OK;
 }
 
-// First part of a reencode: the per-frame work area; an inter frame's refit
-// weight sums of the previous frame's blocks, an intra frame's zeroed
-// completion words.
-mptc_status reencode_begin(mptc_ctx *ctx, const mptc::SearchParams &P, cudaStream_t s) {
-  MPTC_CUDA(cudaMemsetAsync(ctx->work, 0, work_bytes(ctx->ntiles), s));
-  if (P.prev) {
-    mptc::weight_desc_kernel<<<(ctx->nblk + 255) / 256, 256, 0, s>>>(P.prev, ctx->nblk, ctx->wdesc);
-    ctx->launches += 2;  // weight descriptors; the pending compaction follows the search
-  } else {
-    MPTC_CUDA(cudaMemsetAsync(ctx->done, 0, (size_t)ctx->nblk * sizeof(uint64_t), s));
-  }
+// First part of a reencode (see launch_begin).
+mptc_status reencode_begin(mptc_ctx *ctx, const mptc::SearchParams &P, bool chained, cudaStream_t s) {
+  ctx->launches += launch_begin(P, ctx->wdesc, ctx->ntiles, chained, s);
+  if (P.prev) ++ctx->launches;  // the pending compaction, which follows the search
   MPTC_CUDA(cudaGetLastError());
   return MPTC_OK;
 }
@@ -629,9 +661,16 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
     // pending = blocks the inter pass left open, in wavefront order, with
     // the sweeps' first estimates and change flags
     const int sw = sweep_count(ctx->cfg.intra_sweeps);
-    mptc::pending_scan_kernel<<<ctx->ntiles, 256, 0, s>>>(
-        ctx->order, ctx->done, P.stb, ctx->nblk, ctx->ntiles, ctx->tile_state, ctx->work + 10, ctx->pending,
-        ctx->work + 5, ctx->sweep, ctx->sweep + 3 * (size_t)ctx->nblk, sw ? sw + 1 : 0, ctx->work + 1);
+    uint32_t *changed = ctx->sweep + 3 * (size_t)ctx->nblk;
+    const int flags = sw ? sw + 1 : 0;
+    if (ctx->model)  // in a batch behind an event wait
+      mptc::pending_scan_kernel<<<ctx->ntiles, 256, 0, s>>>(ctx->order, ctx->done, P.stb, ctx->nblk, ctx->ntiles,
+                                                           ctx->tile_state, ctx->work + 10, ctx->pending,
+                                                           ctx->work + 5, ctx->sweep, changed, flags, ctx->work + 1);
+    else
+      launch_chain(mptc::pending_scan_kernel, ctx->ntiles, 256, s, ctx->order, ctx->done, P.stb, ctx->nblk,
+                   ctx->ntiles, ctx->tile_state, ctx->work + 10, ctx->pending, ctx->work + 5, ctx->sweep, changed,
+                   flags, ctx->work + 1);
   }
   {
     KernelTimer t(ctx, prev_final_dev ? K_PENDING : K_INTRA, s);
@@ -641,7 +680,7 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
                                            sweep_count(ctx->cfg.intra_sweeps), ctx->sweep_part,
                                            std::min(ctx->nblk, kSweepPartCap), s);
     else
-      ctx->launches += launch_intra_frame(P, ctx->wdesc, ctx->order, ig,
+      ctx->launches += launch_intra_frame(P, ctx->order, ig,
                                           ctx->intra_cap > 0 ? std::min(ctx->intra_cap, ctx->sm_count) : ctx->sm_count,
                                           s);
   }
@@ -649,9 +688,9 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
   const uint16_t *m16 = P.motion;
   {
     KernelTimer t(ctx, K_UNIQUE, s);
-    mptc::unique_scan_kernel<<<ctx->ntiles, 256, 0, s>>>(m16, P.stb, ctx->nblk, ctx->ntiles,
-                                                        ctx->tile_state + ctx->ntiles, ctx->work + 11, unique_dev,
-                                                        n_unique_dev, ctx->work + 2, ctx->work + 1);
+    launch_chain(mptc::unique_scan_kernel, ctx->ntiles, 256, s, m16, P.stb, ctx->nblk, ctx->ntiles,
+                 ctx->tile_state + ctx->ntiles, ctx->work + 11, unique_dev, n_unique_dev, ctx->work + 2,
+                 ctx->work + 1);
     ++ctx->launches;
   }
   MPTC_CUDA(cudaGetLastError());
@@ -797,15 +836,16 @@ mptc_status mptc_dxt1_encode(mptc_ctx *ctx, const uint8_t *rgb_dev, uint64_t *bl
   return MPTC_OK;
 }
 
-mptc_status mptc_reencode(mptc_ctx *ctx, const uint8_t *rgb_dev, const uint64_t *stb_dev, const int32_t *orig_err_dev,
-                          const uint64_t *prev_final_dev, uint64_t *final_dev, uint8_t *motion_dev,
-                          uint32_t *unique_dev, uint32_t *n_unique_dev, void *stream) {
+static mptc_status reencode_run(mptc_ctx *ctx, const uint8_t *rgb_dev, const uint64_t *stb_dev,
+                                const int32_t *orig_err_dev, const uint64_t *prev_final_dev, uint64_t *final_dev,
+                                uint8_t *motion_dev, uint32_t *unique_dev, uint32_t *n_unique_dev, bool chained,
+                                void *stream) {
   mptc_status st = reencode_check(ctx, rgb_dev, stb_dev, orig_err_dev, prev_final_dev, final_dev, motion_dev,
                                   unique_dev, n_unique_dev);
   if (st != MPTC_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const mptc::SearchParams P = make_params(ctx, rgb_dev, stb_dev, orig_err_dev, prev_final_dev, final_dev, motion_dev);
-  st = reencode_begin(ctx, P, s);
+  st = reencode_begin(ctx, P, chained, s);
   if (st != MPTC_OK) return st;
   if (prev_final_dev) {
     if (ctx->model) {
@@ -820,6 +860,13 @@ mptc_status mptc_reencode(mptc_ctx *ctx, const uint8_t *rgb_dev, const uint64_t 
   return reencode_finish(ctx, P, unique_dev, n_unique_dev, s);
 }
 
+mptc_status mptc_reencode(mptc_ctx *ctx, const uint8_t *rgb_dev, const uint64_t *stb_dev, const int32_t *orig_err_dev,
+                          const uint64_t *prev_final_dev, uint64_t *final_dev, uint8_t *motion_dev,
+                          uint32_t *unique_dev, uint32_t *n_unique_dev, void *stream) {
+  return reencode_run(ctx, rgb_dev, stb_dev, orig_err_dev, prev_final_dev, final_dev, motion_dev, unique_dev,
+                      n_unique_dev, false, stream);
+}
+
 mptc_status mptc_encode_frame(mptc_ctx *ctx, const uint8_t *rgb_dev, const uint64_t *prev_final_dev, uint64_t *stb_dev,
                               uint64_t *final_dev, uint8_t *motion_dev, uint32_t *unique_dev, uint32_t *n_unique_dev,
                               void *stream) {
@@ -827,8 +874,8 @@ mptc_status mptc_encode_frame(mptc_ctx *ctx, const uint8_t *rgb_dev, const uint6
   uint64_t *stb = stb_dev ? stb_dev : ctx->stb;
   mptc_status st = mptc_dxt1_encode(ctx, rgb_dev, stb, ctx->orig_err, stream);
   if (st != MPTC_OK) return st;
-  return mptc_reencode(ctx, rgb_dev, stb, ctx->orig_err, prev_final_dev, final_dev, motion_dev, unique_dev,
-                       n_unique_dev, stream);
+  return reencode_run(ctx, rgb_dev, stb, ctx->orig_err, prev_final_dev, final_dev, motion_dev, unique_dev,
+                       n_unique_dev, true, stream);
 }
 
 mptc_status mptc_last_frame_stats(mptc_ctx *ctx, mptc_frame_stats *out, void *stream) {
@@ -897,6 +944,7 @@ mptc_status mptc_encode_frame_host(mptc_ctx *ctx, const uint8_t *rgb_host, int32
 namespace {
 
 __global__ void status_or_kernel(const uint32_t *__restrict__ work, uint32_t *__restrict__ acc) {
+  mptc::depend();
   if (threadIdx.x == 0 && work[1]) atomicOr(acc, work[1]);  // two lanes may report at once
 }
 
@@ -1049,7 +1097,7 @@ static mptc_status encode_stream_host_run(mptc_ctx *ctx, const uint8_t *frames_h
       st = run_inter_frame(ctx, n_inter++, r.rgb[i], r.up[i], prev, r.fin[i], r.motion[i], r.unique[i],
                            r.n_unique[i], s);
     if (st != MPTC_OK) return lane ? fail(ctx, st, std::string("intra lane: ") + b->err) : st;
-    status_or_kernel<<<1, 32, 0, es>>>(lane ? b->work : ctx->work, ctx->run_status);
+    launch_chain(status_or_kernel, 1, 32, es, lane ? b->work : ctx->work, ctx->run_status);
     ++ctx->launches;
     MPTC_CUDA(cudaEventRecord(r.enc[i], es));
     prev_in_lane = lane;
@@ -1112,7 +1160,7 @@ static mptc_status encode_stream_device_run(mptc_ctx *ctx, const uint8_t *frames
       st = mptc_encode_frame(b, in, nullptr, nullptr, fin, motion_dev + 2 * k * n, unique_dev + k * n,
                              n_unique_dev + k, ctx->lane_s);
       if (st != MPTC_OK) return fail(ctx, st, std::string("intra lane: ") + b->err);
-      status_or_kernel<<<1, 32, 0, ctx->lane_s>>>(b->work, ctx->run_status);
+      launch_chain(status_or_kernel, 1, 32, ctx->lane_s, b->work, ctx->run_status);
       ++ctx->launches;
       MPTC_CUDA(cudaEventRecord(ctx->lane_done, ctx->lane_s));
       prev_in_lane = true;
@@ -1126,7 +1174,7 @@ static mptc_status encode_stream_device_run(mptc_ctx *ctx, const uint8_t *frames
         st = run_inter_frame(ctx, n_inter++, in, nullptr, prev, fin, motion_dev + 2 * k * n, unique_dev + k * n,
                              n_unique_dev + k, s);
       if (st != MPTC_OK) return st;
-      status_or_kernel<<<1, 32, 0, s>>>(ctx->work, ctx->run_status);
+      launch_chain(status_or_kernel, 1, 32, s, ctx->work, ctx->run_status);
       ++ctx->launches;
     }
     prev = fin;
@@ -1438,10 +1486,6 @@ extern "C" mptc_status mptc_encode_frame_noalloc(const mptc_config *cfg, int32_t
   const int bw = width / 4, bh = height / 4, n = (int)nblk;
   const int ntiles = (n + mptc::kScanTile - 1) / mptc::kScanTile;
 
-  // The scratch keeps the previous call's contents: clear the counters and
-  // tile states, and the completion flags when no inter pass will write them.
-  if (cudaMemsetAsync(work, 0, work_bytes(ntiles), s) != cudaSuccess) return MPTC_ECUDA;
-  if (!prev_final_dev && cudaMemsetAsync(done, 0, nblk * sizeof(uint64_t), s) != cudaSuccess) return MPTC_ECUDA;
   mptc::wavefront_order_kernel<<<(n + 255) / 256, 256, 0, s>>>(bw, bh, cfg->search_area, order);
   mptc::dxt1_encode_kernel<<<(n + 127) / 128, 128, 0, s>>>(rgb_dev, width, bw, n, stb, orig);
   mptc::SearchParams P;
@@ -1460,20 +1504,21 @@ extern "C" mptc_status mptc_encode_frame_noalloc(const mptc_config *cfg, int32_t
   P.bh = bh;
   P.sa = cfg->search_area;
   P.thr = cfg->err_threshold;
+  // the scratch keeps the previous call's contents: launch_begin clears the
+  // counters and tile states, and the completion flags that no inter pass writes
+  launch_begin(P, wdesc, ntiles, true, s);
   if (prev_final_dev) {
-    mptc::weight_desc_kernel<<<(n + 255) / 256, 256, 0, s>>>(prev_final_dev, n, wdesc);
     launch_inter_search(P, kSearchWarps, work, pend, d->sm_count, s);
     const int sw = sweep_count(cfg->intra_sweeps);
-    mptc::pending_scan_kernel<<<ntiles, 256, 0, s>>>(order, done, stb, n, ntiles, tile_state, work + 10, pend,
-                                                    work + 5, sweep, sweep + 3 * (size_t)n, sw ? sw + 1 : 0,
-                                                    work + 1);
+    launch_chain(mptc::pending_scan_kernel, ntiles, 256, s, order, done, stb, n, ntiles, tile_state, work + 10, pend,
+                 work + 5, sweep, sweep + 3 * (size_t)n, sw ? sw + 1 : 0, work + 1);
     launch_intra_sweeps(P, pend, work + 5, sweep, n, d->intra_grid, sw, sweep_part, kSweepPartCapNoalloc, s);
   } else {
-    launch_intra_frame(P, wdesc, order, d->intra_grid, d->sm_count, s);
+    launch_intra_frame(P, order, d->intra_grid, d->sm_count, s);
   }
   const uint16_t *m16 = reinterpret_cast<const uint16_t *>(motion_dev);
-  mptc::unique_scan_kernel<<<ntiles, 256, 0, s>>>(m16, stb, n, ntiles, tile_state + ntiles, work + 11, unique_dev,
-                                                  n_unique_dev, work + 2, work + 1);
+  launch_chain(mptc::unique_scan_kernel, ntiles, 256, s, m16, stb, n, ntiles, tile_state + ntiles, work + 11,
+               unique_dev, n_unique_dev, work + 2, work + 1);
   noalloc_status_kernel<<<1, 32, 0, s>>>(work, n_unique_dev);
   return cudaGetLastError() == cudaSuccess ? MPTC_OK : MPTC_ECUDA;
 }
@@ -1532,7 +1577,7 @@ mptc_status batch_launch(mptc_batch *b, const int32_t *is_intra, int parity, cud
     mptc_status st = mptc_dxt1_encode(c, b->rgb[i], c->stb, c->orig_err, si);
     if (st != MPTC_OK) return st;
     P[i] = make_params(c, b->rgb[i], c->stb, c->orig_err, prev, b->fin[parity][i], b->motion[i]);
-    st = reencode_begin(c, P[i], si);
+    st = reencode_begin(c, P[i], false, si);
     if (st != MPTC_OK) return st;
     if (prev && !c->model) {
       KernelTimer t(c, K_INTER, si);
@@ -1644,7 +1689,7 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
       mptc_status st = mptc_encode_frame(c->lane_b, frames[i] + k * n * 48, nullptr, nullptr, fin[i] + k * n,
                                          mot[i] + 2 * k * n, uni[i] + k * n, n_uni[i] + k, c->lane_s);
       if (st != MPTC_OK) return st;
-      status_or_kernel<<<1, 32, 0, c->lane_s>>>(c->lane_b->work, b->run_status);
+      launch_chain(status_or_kernel, 1, 32, c->lane_s, c->lane_b->work, b->run_status);
       if (cudaEventRecord(b->lane_ev[i][k], c->lane_s) != cudaSuccess) return MPTC_ECUDA;
     }
   }
@@ -1677,7 +1722,7 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
           cudaStreamWaitEvent(si, c->stb_done[j], 0) != cudaSuccess)
         return MPTC_ECUDA;
       P[i] = make_params(c, in, c->stb_slot[j], c->orig_slot[j], prev, fin[i] + k * n, mot[i] + 2 * k * n);
-      st = reencode_begin(c, P[i], si);
+      st = reencode_begin(c, P[i], false, si);
       if (st != MPTC_OK) return st;
       if (c->model) {
         jobs.push_back(LearnedJob{c, P[i]});
@@ -1708,7 +1753,7 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
       if (c->model && !jobs.empty() && cudaStreamWaitEvent(si, b->learned_ev, 0) != cudaSuccess) return MPTC_ECUDA;
       mptc_status st = reencode_finish(c, P[i], uni[i] + k * n, n_uni[i] + k, si);
       if (st != MPTC_OK) return st;
-      status_or_kernel<<<1, 32, 0, si>>>(c->work, b->run_status);
+      launch_chain(status_or_kernel, 1, 32, si, c->work, b->run_status);
       if (cudaEventRecord(c->stb_free[slot[i]], si) != cudaSuccess) return MPTC_ECUDA;
     }
   }

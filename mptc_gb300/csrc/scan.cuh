@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(256) pending_scan_kernel(const uint32_t *__res
                                                            uint32_t *__restrict__ n_pending,
                                                            uint32_t *__restrict__ cur, uint32_t *__restrict__ changed,
                                                            int n_flags, uint32_t *status) {
+  depend();
+  release_next();
   __shared__ int s_tile;
   __shared__ uint32_t s_warp[8], s_before;
   if (threadIdx.x == 0) s_tile = (int)atomicAdd(claim, 1u);
@@ -129,6 +131,8 @@ __global__ void __launch_bounds__(256) unique_scan_kernel(const uint16_t *__rest
                                                           uint32_t *__restrict__ unique,
                                                           uint32_t *__restrict__ n_unique,
                                                           uint32_t *__restrict__ stats, uint32_t *status) {
+  depend();
+  release_next();
   __shared__ int s_tile;
   __shared__ uint32_t s_warp[8], s_before;
   if (threadIdx.x == 0) s_tile = (int)atomicAdd(claim, 1u);
