@@ -1,5 +1,5 @@
 // Completion words and their bounded waits: the memory-order helpers the
-// intra dataflow and the scans use, and the intra wavefront order.
+// intra dataflow and the scans use.
 #pragma once
 #include <cstdint>
 
@@ -58,30 +58,6 @@ __device__ __forceinline__ uint64_t wait_done(const uint64_t *done, size_t idx, 
   }
   atomicOr(status, kDevTimeout);
   return 0;
-}
-
-// Wavefront order of the intra dataflow. Block (x, y) reads, in this frame,
-// only blocks of rows y-2sa+1 .. y-1 with columns up to x+sa-1 and blocks of
-// row y left of x; with t = x + sa*y every such block has a smaller t. Blocks
-// are therefore ranked by (t, y): order[rank] = block index. Blocks of equal t
-// never read each other.
-__global__ void __launch_bounds__(256) wavefront_order_kernel(int bw, int bh, int sa, uint32_t *__restrict__ order) {
-  const int n = bw * bh;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-    const int y = idx / bw, x = idx - y * bw;
-    const long long t = (long long)x + (long long)sa * y;
-    long long rank = 0;
-    for (int yy = 0; yy < bh; ++yy) {  // blocks with t' < t: x' < t - sa*y'
-      const long long c = t - (long long)sa * yy;
-      if (c <= 0) break;
-      rank += c < bw ? c : bw;
-    }
-    for (int yy = 0; yy < y; ++yy) {  // blocks with t' == t and y' < y
-      const long long xp = t - (long long)sa * yy;
-      rank += (xp >= 0 && xp < bw);
-    }
-    order[rank] = (uint32_t)idx;
-  }
 }
 
 }  // namespace mptc

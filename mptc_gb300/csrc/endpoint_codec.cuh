@@ -13,17 +13,17 @@
 // arithmetic (decoder.cpp:24-41, 109-201), and the index words from the motion
 // codes (decoder.cpp:203-254): unique blocks take the next palette entry in
 // raster order, inter blocks copy from the previous frame, intra blocks copy
-// from an earlier block of the same frame. The intra copies form chains; they
-// are resolved by pointer jumping (log2(blocks) rounds) instead of the
-// reference's raster loop.
+// from an earlier block of the same frame. The intra copies form chains that
+// every block follows by itself, shortening them for the others on the way,
+// instead of the reference's raster loop.
 //
-// Forward: one CTA per (64x64 tile, plane), two int16 tiles in shared memory
-// (source and destination of each lifting pass). Inverse: one CTA per
-// (tile, endpoint) with its three planes (2 x 24 KiB), which the RGB565
-// conversion needs together.
+// Both transforms: one CTA per (64x64 tile, plane), two int16 tiles in shared
+// memory (source and destination of each lifting pass).
 #pragma once
 
 #include <cstdint>
+
+#include "lookback.cuh"
 
 namespace mptc {
 
@@ -31,242 +31,388 @@ constexpr int kTile = 64;                 // endpoint tile edge (blocks)
 constexpr int kTileElems = kTile * kTile;
 constexpr int kCodecThreads = 256;
 
-// Mirror index into [0, len) for the indices the lifting uses (-1 and len).
-__device__ __forceinline__ int lift_mirror(int i, int len) { return i < 0 ? -i : (i >= len ? 2 * len - 2 - i : i); }
+// The lifting passes. What bounds them is latency: a tile is 12 dependent
+// passes (two per level) and a frame has few tiles (240 planes at 2048x1280, at
+// most two per SM), so a pass has to be short: each thread takes a piece of
+// K outputs of each half of a line into registers and computes its
+// halo's details itself, one barrier a pass; the levels up to 16x16 are one
+// warp's work and need none. Rows of 66 elements (33 words) keep both
+// directions free of bank conflicts: a row pass has its lanes in a column, a
+// column pass takes two adjacent columns per lane as one word.
+// One thread per output, two steps and barriers a pass, took 31 us for a
+// 2048x1280 frame forward and 52 inverse; now 7.6 us forward, and 11.5 inverse
+// together with the motion codes.
+constexpr int kPitch = kTile + 2;
+struct __align__(16) LiftTile {
+  uint32_t w[kTile * kPitch / 2];
+};
 
-// One forward lifting pass over `lines` lines of length `len` (power of two)
-// of `planes` planes: element k of line l of plane p is at
-// p*kTileElems + l*lstride + k*estride. src -> dst, details in the upper half
-// (codec/wavelet.cpp:30-66).
-__device__ __forceinline__ void forward_pass(const int16_t *src, int16_t *dst, int planes, int len, int lstride,
-                                             int estride) {
-  const int half = len >> 1;  // len is even: mid point == half
-  const int work = planes * len * half;
-  for (int w = threadIdx.x; w < work; w += blockDim.x) {
-    const int p = w / (len * half), r = w - p * len * half;
-    const int l = r / half, k = r - l * half;
-    const int16_t *s = src + p * kTileElems + l * lstride;
-    const int i = 2 * k + 1;
-    dst[p * kTileElems + l * lstride + (half + k) * estride] =
-        (int16_t)(s[i * estride] - (s[(i - 1) * estride] + s[lift_mirror(i + 1, len) * estride]) / 2);
+__device__ __forceinline__ int lo16(uint32_t w) { return (int)(int16_t)(w & 0xFFFFu); }
+__device__ __forceinline__ int hi16(uint32_t w) { return (int)(int16_t)(w >> 16); }
+__device__ __forceinline__ uint32_t pack16(int lo, int hi) { return ((uint32_t)lo & 0xFFFFu) | ((uint32_t)hi << 16); }
+
+// A piece of a forward line (codec/wavelet.cpp:30-66): e[2 + i] = element i of
+// the piece, i = -2 .. 2K (the halo unread where the line ends); details
+// hi[k] = e[2k+1] - (e[2k] + e[2k+2]) / 2, approximations lo[k] = e[2k] +
+// (hi[k-1] + hi[k] + 2) / 4, mirrored at both ends, each stored in 16 bits.
+template <int K>
+__device__ __forceinline__ void forward_piece(int (&e)[2 * K + 3], bool first, bool last, int (&lo)[K], int (&hi)[K]) {
+  if (last) e[2 * K + 2] = e[2 * K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) hi[k] = (int)(int16_t)(e[2 * k + 3] - (e[2 * k + 2] + e[2 * k + 4]) / 2);
+  int before = first ? hi[0] : (int)(int16_t)(e[1] - (e[0] + e[2]) / 2);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    lo[k] = (int)(int16_t)(e[2 * k + 2] + (before + hi[k] + 2) / 4);
+    before = hi[k];
   }
-  __syncthreads();
-  for (int w = threadIdx.x; w < work; w += blockDim.x) {
-    const int p = w / (len * half), r = w - p * len * half;
-    const int l = r / half, k = r - l * half;
-    const int16_t *s = src + p * kTileElems + l * lstride;
-    int16_t *d = dst + p * kTileElems + l * lstride;
-    const int i = 2 * k;
-    const int prev = half + lift_mirror(i - 1, len) / 2, next = half + (i + 1) / 2;
-    d[k * estride] = (int16_t)(s[i * estride] + (d[prev * estride] + d[next * estride] + 2) / 4);
-  }
-  __syncthreads();
 }
 
-// Inverse of forward_pass (codec/wavelet.cpp:69-99).
-__device__ __forceinline__ void inverse_pass(const int16_t *src, int16_t *dst, int len, int lstride, int estride) {
-  const int half = len >> 1;
-  const int work = 3 * len * half;
-  for (int w = threadIdx.x; w < work; w += blockDim.x) {
-    const int p = w / (len * half), r = w - p * len * half;
-    const int l = r / half, k = r - l * half;
-    const int16_t *s = src + p * kTileElems + l * lstride;
-    const int i = 2 * k;
-    const int prev = half + lift_mirror(i - 1, len) / 2, next = half + (i + 1) / 2;
-    dst[p * kTileElems + l * lstride + i * estride] =
-        (int16_t)(s[k * estride] - (s[prev * estride] + s[next * estride] + 2) / 4);
+// Its inverse (codec/wavelet.cpp:69-99): s[k] = approximation k of the piece (k
+// = 0 .. K), d[1 + k] = detail k (k = -1 .. K); even and odd elements.
+template <int K>
+__device__ __forceinline__ void inverse_piece(int (&s)[K + 1], int (&d)[K + 2], bool first, bool last, int (&even)[K],
+                                              int (&odd)[K]) {
+  if (first) d[0] = d[1];
+#pragma unroll
+  for (int k = 0; k < K; ++k) even[k] = (int)(int16_t)(s[k] - (d[k] + d[k + 1] + 2) / 4);
+  const int after = last ? even[K - 1] : (int)(int16_t)(s[K] - (d[K] + d[K + 1] + 2) / 4);
+#pragma unroll
+  for (int k = 0; k < K; ++k) odd[k] = (int)(int16_t)(d[k + 1] + (even[k] + (k + 1 < K ? even[k + 1] : after)) / 2);
+}
+
+// One pass over the top-left DIM x DIM corner, src -> dst, by `threads` threads.
+template <int DIM, int K>
+__device__ __forceinline__ void forward_rows(const LiftTile &src, LiftTile &dst, int tid, int threads) {
+  constexpr int kHalf = DIM / 2, kPieces = kHalf / K;
+  int16_t *out = reinterpret_cast<int16_t *>(dst.w);
+  for (int t = tid; t < DIM * kPieces; t += threads) {
+    const int row = t % DIM, k0 = t / DIM * K;
+    const uint32_t *in = src.w + row * (kPitch / 2);
+    int e[2 * K + 3], lo[K], hi[K];
+    const uint32_t left = in[max(k0 - 1, 0)];
+    e[0] = lo16(left), e[1] = hi16(left);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const uint32_t w = in[k0 + k];
+      e[2 * k + 2] = lo16(w), e[2 * k + 3] = hi16(w);
+    }
+    e[2 * K + 2] = lo16(in[min(k0 + K, kHalf - 1)]);
+    forward_piece<K>(e, k0 == 0, k0 + K == kHalf, lo, hi);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      out[row * kPitch + k0 + k] = (int16_t)lo[k];
+      out[row * kPitch + kHalf + k0 + k] = (int16_t)hi[k];
+    }
   }
-  __syncthreads();
-  for (int w = threadIdx.x; w < work; w += blockDim.x) {
-    const int p = w / (len * half), r = w - p * len * half;
-    const int l = r / half, k = r - l * half;
-    const int16_t *s = src + p * kTileElems + l * lstride;
-    int16_t *d = dst + p * kTileElems + l * lstride;
-    const int i = 2 * k + 1;
-    d[i * estride] = (int16_t)(s[(half + k) * estride] + (d[(i - 1) * estride] + d[lift_mirror(i + 1, len) * estride]) / 2);
+}
+
+template <int DIM, int K>
+__device__ __forceinline__ void forward_columns(const LiftTile &src, LiftTile &dst, int tid, int threads) {
+  constexpr int kHalf = DIM / 2, kPieces = kHalf / K, kRow = kPitch / 2;
+  for (int t = tid; t < kHalf * kPieces; t += threads) {  // kHalf column pairs
+    const int c = t % kHalf, k0 = t / kHalf * K;
+    const uint32_t *in = src.w + c;
+    int e[2 * K + 3], f[2 * K + 3], lo[K], hi[K], lo2[K], hi2[K];
+#pragma unroll
+    for (int i = 0; i < 2 * K + 3; ++i) {
+      const uint32_t w = in[min(max(2 * k0 - 2 + i, 0), DIM - 1) * kRow];
+      e[i] = lo16(w), f[i] = hi16(w);
+    }
+    forward_piece<K>(e, k0 == 0, k0 + K == kHalf, lo, hi);
+    forward_piece<K>(f, k0 == 0, k0 + K == kHalf, lo2, hi2);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      dst.w[(k0 + k) * kRow + c] = pack16(lo[k], lo2[k]);
+      dst.w[(kHalf + k0 + k) * kRow + c] = pack16(hi[k], hi2[k]);
+    }
   }
-  __syncthreads();
+}
+
+template <int DIM, int K>
+__device__ __forceinline__ void inverse_rows(const LiftTile &src, LiftTile &dst, int tid, int threads) {
+  constexpr int kHalf = DIM / 2, kPieces = kHalf / K;
+  const int16_t *in = reinterpret_cast<const int16_t *>(src.w);
+  for (int t = tid; t < DIM * kPieces; t += threads) {
+    const int row = t % DIM, k0 = t / DIM * K;
+    const int16_t *a = in + row * kPitch;
+    int s[K + 1], d[K + 2], even[K], odd[K];
+#pragma unroll
+    for (int k = 0; k <= K; ++k) s[k] = a[min(k0 + k, kHalf - 1)];
+#pragma unroll
+    for (int k = 0; k < K + 2; ++k) d[k] = a[kHalf + min(max(k0 - 1 + k, 0), kHalf - 1)];
+    inverse_piece<K>(s, d, k0 == 0, k0 + K == kHalf, even, odd);
+#pragma unroll
+    for (int k = 0; k < K; ++k) dst.w[row * (kPitch / 2) + k0 + k] = pack16(even[k], odd[k]);
+  }
+}
+
+template <int DIM, int K>
+__device__ __forceinline__ void inverse_columns(const LiftTile &src, LiftTile &dst, int tid, int threads) {
+  constexpr int kHalf = DIM / 2, kPieces = kHalf / K, kRow = kPitch / 2;
+  for (int t = tid; t < kHalf * kPieces; t += threads) {
+    const int c = t % kHalf, k0 = t / kHalf * K;
+    const uint32_t *in = src.w + c;
+    int s[K + 1], d[K + 2], even[K], odd[K], s2[K + 1], d2[K + 2], even2[K], odd2[K];
+#pragma unroll
+    for (int k = 0; k <= K; ++k) {
+      const uint32_t w = in[min(k0 + k, kHalf - 1) * kRow];
+      s[k] = lo16(w), s2[k] = hi16(w);
+    }
+#pragma unroll
+    for (int k = 0; k < K + 2; ++k) {
+      const uint32_t w = in[(kHalf + min(max(k0 - 1 + k, 0), kHalf - 1)) * kRow];
+      d[k] = lo16(w), d2[k] = hi16(w);
+    }
+    inverse_piece<K>(s, d, k0 == 0, k0 + K == kHalf, even, odd);
+    inverse_piece<K>(s2, d2, k0 == 0, k0 + K == kHalf, even2, odd2);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      dst.w[(2 * (k0 + k)) * kRow + c] = pack16(even[k], even2[k]);
+      dst.w[(2 * (k0 + k) + 1) * kRow + c] = pack16(odd[k], odd2[k]);
+    }
+  }
 }
 
 // grid (bw/64, bh/64, 6 planes: Y, Co, Cg of endpoint 1, then of endpoint 2),
 // one plane of one tile per CTA. coeff: 6 planes of bw*bh bytes,
-// [Y1 | Co1 | Cg1 | Y2 | Co2 | Cg2], each plane raster order over the image.
+// [Y1 | Co1 | Cg1 | Y2 | Co2 | Cg2], each plane raster order over the image;
+// written in words where it is aligned to them (bw is a multiple of 64).
 __global__ void __launch_bounds__(kCodecThreads) endpoint_forward_kernel(const uint64_t *__restrict__ blocks, int bw,
                                                                          int bh, uint8_t *__restrict__ coeff) {
-  __shared__ int16_t a[kTileElems], b[kTileElems];
-  const int tx = blockIdx.x * kTile, ty = blockIdx.y * kTile, plane = blockIdx.z;
+  __shared__ LiftTile a, b;
+  depend();
+  release_next();
+  const int tid = threadIdx.x, tx = blockIdx.x * kTile, ty = blockIdx.y * kTile, plane = blockIdx.z;
   const int ep = plane / 3, channel = plane - 3 * ep;
   const size_t n = (size_t)bw * bh;
-  for (int e = threadIdx.x; e < kTileElems; e += blockDim.x) {
-    const int y = e >> 6, x = e & 63;
-    const uint32_t lo = (uint32_t)blocks[(size_t)(ty + y) * bw + tx + x];
+  const uint32_t *src = reinterpret_cast<const uint32_t *>(blocks + (size_t)ty * bw + tx);
+  int16_t *a16 = reinterpret_cast<int16_t *>(a.w);
+#pragma unroll
+  for (int r = 0; r < kTileElems / kCodecThreads; ++r) {
+    const int e = r * kCodecThreads + tid, y = e >> 6, x = e & 63;
+    const uint32_t lo = src[2 * ((size_t)y * bw + x)];
     const int c = (int)(ep ? (lo >> 16) : (lo & 0xFFFFu));
     const int r5 = c >> 11, g6 = (c >> 5) & 63, b5 = c & 31;
     const int co = r5 - b5, t = r5 + b5 + (b5 >> 4), cg = g6 - t;
-    a[e] = (int16_t)(channel == 0 ? t + cg / 2 : (channel == 1 ? co : cg));
+    a16[y * kPitch + x] = (int16_t)(channel == 0 ? t + cg / 2 : (channel == 1 ? co : cg));
   }
   __syncthreads();
-  for (int dim = kTile; dim > 1; dim >>= 1) {
-    forward_pass(a, b, 1, dim, 1, kTile);   // columns: line = column, element stride = row
-    forward_pass(b, a, 1, dim, kTile, 1);   // rows
+  forward_columns<64, 4>(a, b, tid, kCodecThreads);
+  __syncthreads();
+  forward_rows<64, 8>(b, a, tid, kCodecThreads);
+  __syncthreads();
+  forward_columns<32, 2>(a, b, tid, kCodecThreads);
+  __syncthreads();
+  forward_rows<32, 2>(b, a, tid, kCodecThreads);
+  __syncthreads();
+  if (tid < 32) {
+    forward_columns<16, 2>(a, b, tid, 32);
+    __syncwarp();
+    forward_rows<16, 4>(b, a, tid, 32);
+    __syncwarp();
+    forward_columns<8, 1>(a, b, tid, 32);
+    __syncwarp();
+    forward_rows<8, 1>(b, a, tid, 32);
+    __syncwarp();
+    forward_columns<4, 1>(a, b, tid, 32);
+    __syncwarp();
+    forward_rows<4, 1>(b, a, tid, 32);
+    __syncwarp();
+    forward_columns<2, 1>(a, b, tid, 32);
+    __syncwarp();
+    forward_rows<2, 1>(b, a, tid, 32);
   }
-  uint8_t *out = coeff + (size_t)plane * n;
-  for (int e = threadIdx.x; e < kTileElems; e += blockDim.x) {
-    const int y = e >> 6, x = e & 63;
-    out[(size_t)(ty + y) * bw + tx + x] = (uint8_t)((int)(int8_t)a[e] + 128);
+  __syncthreads();
+  uint8_t *out = coeff + (size_t)plane * n + (size_t)ty * bw + tx;
+  const bool words = (reinterpret_cast<uintptr_t>(coeff) & 3u) == 0;
+#pragma unroll
+  for (int r = 0; r < kTileElems / 4 / kCodecThreads; ++r) {
+    const int e = r * kCodecThreads + tid, y = e >> 4, x = 4 * (e & 15);
+    const uint32_t w0 = a.w[(y * kPitch + x) / 2], w1 = a.w[(y * kPitch + x) / 2 + 1];
+    // the coefficients wrap to int8 and are offset by 128
+    const uint32_t v = __byte_perm(w0, w1, 0x6420) ^ 0x80808080u;
+    uint8_t *o = out + (size_t)y * bw + x;
+    if (words) {
+      *reinterpret_cast<uint32_t *>(o) = v;
+    } else {
+      o[0] = (uint8_t)v, o[1] = (uint8_t)(v >> 8), o[2] = (uint8_t)(v >> 16), o[3] = (uint8_t)(v >> 24);
+    }
   }
 }
 
-// grid (bw/64, bh/64, 2 endpoints): coefficients -> RGB565 endpoint words.
-__global__ void __launch_bounds__(kCodecThreads) endpoint_inverse_kernel(const uint8_t *__restrict__ coeff, int bw,
-                                                                         int bh, uint16_t *__restrict__ ep_out) {
-  __shared__ int16_t a[3 * kTileElems], b[3 * kTileElems];
-  const int tx = blockIdx.x * kTile, ty = blockIdx.y * kTile, ep = blockIdx.z;
-  const size_t n = (size_t)bw * bh;
-  for (int e = threadIdx.x; e < 3 * kTileElems; e += blockDim.x) {
-    const int p = e >> 12, q = e & (kTileElems - 1), y = q >> 6, x = q & 63;
-    a[e] = (int16_t)((int)coeff[(size_t)(3 * ep + p) * n + (size_t)(ty + y) * bw + tx + x] - 128);
+// One plane of one tile: coefficients -> the plane's values in int8 (planes:
+// as coeff), by one CTA. Where coeff is aligned to words it is read in words.
+__device__ __forceinline__ void inverse_tile(const uint8_t *__restrict__ coeff, int bw, size_t off, LiftTile &a,
+                                             LiftTile &b, uint8_t *__restrict__ planes) {
+  const int tid = threadIdx.x;
+  const bool words = (reinterpret_cast<uintptr_t>(coeff) & 3u) == 0;
+#pragma unroll
+  for (int r = 0; r < kTileElems / 4 / kCodecThreads; ++r) {
+    const int e = r * kCodecThreads + tid, y = e >> 4, x = 4 * (e & 15);
+    const uint8_t *i = coeff + off + (size_t)y * bw + x;
+    uint32_t v;
+    if (words)
+      v = *reinterpret_cast<const uint32_t *>(i);
+    else
+      v = i[0] | (uint32_t)i[1] << 8 | (uint32_t)i[2] << 16 | (uint32_t)i[3] << 24;
+    uint32_t *o = a.w + (y * kPitch + x) / 2;
+    o[0] = pack16((int)(v & 255u) - 128, (int)(v >> 8 & 255u) - 128);
+    o[1] = pack16((int)(v >> 16 & 255u) - 128, (int)(v >> 24) - 128);
   }
   __syncthreads();
-  for (int dim = 2; dim <= kTile; dim <<= 1) {
-    inverse_pass(a, b, dim, kTile, 1);      // rows
-    inverse_pass(b, a, dim, 1, kTile);      // columns
+  if (tid < 32) {
+    inverse_rows<2, 1>(a, b, tid, 32);
+    __syncwarp();
+    inverse_columns<2, 1>(b, a, tid, 32);
+    __syncwarp();
+    inverse_rows<4, 1>(a, b, tid, 32);
+    __syncwarp();
+    inverse_columns<4, 1>(b, a, tid, 32);
+    __syncwarp();
+    inverse_rows<8, 1>(a, b, tid, 32);
+    __syncwarp();
+    inverse_columns<8, 1>(b, a, tid, 32);
+    __syncwarp();
+    inverse_rows<16, 4>(a, b, tid, 32);
+    __syncwarp();
+    inverse_columns<16, 2>(b, a, tid, 32);
   }
-  for (int e = threadIdx.x; e < kTileElems; e += blockDim.x) {
-    const int y = e >> 6, x = e & 63;
-    // int8 arithmetic as the reference stores it (decoder.cpp:24-41, 145-160)
-    const int8_t Y = (int8_t)a[e], Co = (int8_t)a[kTileElems + e], Cg = (int8_t)a[2 * kTileElems + e];
-    const int8_t t = (int8_t)(Y - Cg / 2);
-    const int8_t g = (int8_t)(Cg + t);
-    const int8_t bb = (int8_t)((t - Co) / 2);
-    const int8_t r = (int8_t)(bb + Co);
-    uint16_t w = (uint16_t)(int16_t)r;
-    w = (uint16_t)(w << 6);
-    w |= (uint16_t)(int16_t)g;
-    w = (uint16_t)(w << 5);
-    w |= (uint16_t)(int16_t)bb;
-    ep_out[(size_t)ep * n + (size_t)(ty + y) * bw + tx + x] = w;
+  __syncthreads();
+  inverse_rows<32, 2>(a, b, tid, kCodecThreads);
+  __syncthreads();
+  inverse_columns<32, 2>(b, a, tid, kCodecThreads);
+  __syncthreads();
+  inverse_rows<64, 8>(a, b, tid, kCodecThreads);
+  __syncthreads();
+  inverse_columns<64, 4>(b, a, tid, kCodecThreads);
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kTileElems / 4 / kCodecThreads; ++r) {
+    const int e = r * kCodecThreads + tid, y = e >> 4, x = 4 * (e & 15);
+    const uint32_t *i = a.w + (y * kPitch + x) / 2;
+    *reinterpret_cast<uint32_t *>(planes + off + (size_t)y * bw + x) = __byte_perm(i[0], i[1], 0x6420);
   }
+}
+
+// One endpoint word from its plane values, in the int8 arithmetic in which the
+// reference stores them (decoder.cpp:24-41, 145-160).
+__device__ __forceinline__ uint16_t endpoint_word(uint8_t y, uint8_t o, uint8_t c) {
+  const int8_t Y = (int8_t)y, Co = (int8_t)o, Cg = (int8_t)c;
+  const int8_t t = (int8_t)(Y - Cg / 2);
+  const int8_t g = (int8_t)(Cg + t);
+  const int8_t bb = (int8_t)((t - Co) / 2);
+  const int8_t r = (int8_t)(bb + Co);
+  uint16_t w = (uint16_t)(int16_t)r;
+  w = (uint16_t)(w << 6);
+  w |= (uint16_t)(int16_t)g;
+  w = (uint16_t)(w << 5);
+  w |= (uint16_t)(int16_t)bb;
+  return w;
 }
 
 // --- index words from motion codes ---
 
-constexpr int kDecTile = 1024;  // blocks per CTA of the unique-rank scan
 constexpr uint32_t kDecBadRef = 1u, kDecBadUnique = 2u;
 
-// Classifies blocks: ptr = source block of an intra copy (-1 when resolved),
-// val = index word when resolved (inter copy). Counts unique blocks per tile.
-__global__ void __launch_bounds__(256) decode_classify_kernel(const uint8_t *__restrict__ motion,
-                                                              const uint64_t *__restrict__ prev, int bw, int nblk,
-                                                              int sa, int32_t *__restrict__ ptr,
-                                                              uint32_t *__restrict__ val,
-                                                              uint32_t *__restrict__ tile_counts,
-                                                              uint32_t *__restrict__ err) {
-  const int t0 = blockIdx.x * kDecTile;
-  int c = 0;
-  for (int i = t0 + threadIdx.x; i < min(nblk, t0 + kDecTile); i += blockDim.x) {
+// A block's link: kLinkWord | its index word, or the earlier block that it copies.
+constexpr uint64_t kLinkWord = 1ull << 32;
+
+// First kernel of a frame. The first ntiles CTAs read the motion codes of
+// kScanTile blocks each (tiles taken in order from *claim): a unique block takes
+// palette[its rank among the unique blocks in raster order] (one-pass compaction,
+// lookback.cuh), an inter block the previous frame's word, an intra block a link. The
+// other CTAs are the inverse transform of the frame's tiles, which runs beside
+// them. 11.5 us at 2048x1280; as three kernels, one after
+// another, 52, 5 and 11 us.
+__global__ void __launch_bounds__(kCodecThreads) decode_parts_kernel(
+    const uint8_t *__restrict__ coeff, int bw, int bh, uint8_t *__restrict__ planes,
+    const uint8_t *__restrict__ motion, const uint64_t *prev, int sa, const uint32_t *__restrict__ palette,
+    uint32_t n_unique, int ntiles, uint64_t *state, uint32_t *claim, uint64_t *__restrict__ link,
+    uint32_t *__restrict__ err, uint32_t *__restrict__ status) {
+  __shared__ LiftTile a, b;
+  __shared__ int s_tile;
+  __shared__ uint32_t s_warp[8], s_before;
+  depend();
+  release_next();
+  const int nblk = bw * bh, tid = threadIdx.x;
+  if ((int)blockIdx.x >= ntiles) {
+    const int tiles_x = bw / kTile, tiles = tiles_x * (bh / kTile);
+    const int u = blockIdx.x - ntiles, plane = u / tiles, tile = u - plane * tiles;
+    const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
+    inverse_tile(coeff, bw, (size_t)plane * nblk + (size_t)ty * kTile * bw + tx * kTile, a, b, planes);
+    return;
+  }
+  if (tid == 0) s_tile = (int)atomicAdd(claim, 1u);
+  __syncthreads();
+  const int tile = s_tile, i0 = tile * kScanTile + 4 * tid;
+  unsigned uq = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = i0 + q;
+    if (i >= nblk) break;
     const int x = motion[2 * i], y = motion[2 * i + 1];
-    const int bx = i % bw, by = i / bw;
+    const int by = i / bw, bx = i - by * bw;
     if (x == 255 && y == 255) {
-      ++c;
-      ptr[i] = -1;
-      val[i] = 0;
+      uq |= 1u << q;
     } else if ((x & 0x80) && (y & 0x80)) {
       // linear index as the reference computes it (decoder.cpp:224-236)
       const long ref = (long)(by + (y & 0x7F) - sa) * bw + bx + (x & 0x7F) - sa;
       uint32_t v = 0;
       if (prev && ref >= 0 && ref < nblk) v = (uint32_t)(prev[ref] >> 32);
       else atomicOr(err, kDecBadRef);
-      ptr[i] = -1;
-      val[i] = v;
+      link[i] = kLinkWord | v;
     } else {
       const long ref = (long)(by + y - 2 * sa + 1) * bw + bx + x - sa;
       if (ref >= 0 && ref < i) {
-        ptr[i] = (int32_t)ref;
+        link[i] = (uint64_t)ref;
       } else {
         atomicOr(err, kDecBadRef);
-        ptr[i] = -1;
+        link[i] = kLinkWord;
       }
-      val[i] = 0;
     }
   }
-  c = __reduce_add_sync(0xFFFFFFFFu, c);
-  __shared__ int s[8];
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < 8; ++w) t += s[w];
-    tile_counts[blockIdx.x] = (uint32_t)t;
-  }
-}
-
-// Unique blocks take palette[rank], rank = unique blocks before them in raster order.
-__global__ void __launch_bounds__(256) decode_unique_kernel(const uint8_t *__restrict__ motion, int nblk,
-                                                            const uint32_t *__restrict__ tile_counts,
-                                                            const uint32_t *__restrict__ palette, uint32_t n_unique,
-                                                            uint32_t *__restrict__ val, uint32_t *__restrict__ err) {
-  __shared__ uint32_t s_base, s_warp[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    uint32_t b = 0, total = 0;
-    for (int t = 0; t < (int)gridDim.x; ++t) {
-      if (t < (int)blockIdx.x) b += tile_counts[t];
-      total += tile_counts[t];
-    }
-    s_base = b;
-    if (blockIdx.x == 0 && total != n_unique) atomicOr(err, kDecBadUnique);
+  uint32_t total;
+  uint32_t off = cta_exclusive_scan(__popc(uq), s_warp, total);
+  if (tid < 32) {
+    const uint32_t before = lookback(state, tile, total, status);
+    if (tid == 0) s_before = before;
   }
   __syncthreads();
-  const int t0 = blockIdx.x * kDecTile, t1 = min(nblk, t0 + kDecTile);
-  for (int c0 = t0; c0 < t1; c0 += 256) {
-    const int i = c0 + threadIdx.x;
-    const bool u = i < t1 && motion[2 * i] == 255 && motion[2 * i + 1] == 255;
-    const unsigned bal = __ballot_sync(0xFFFFFFFFu, u);
-    if (lane == 0) s_warp[warp] = __popc(bal);
-    __syncthreads();
-    uint32_t off = s_base;
-    for (int w = 0; w < warp; ++w) off += s_warp[w];
-    off += __popc(bal & ((1u << lane) - 1u));
-    if (u) val[i] = off < n_unique ? palette[off] : 0u;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t t = 0;
-      for (int w = 0; w < 8; ++w) t += s_warp[w];
-      s_base += t;
+  off += s_before;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if ((uq >> q) & 1u) {
+      link[i0 + q] = kLinkWord | (off < n_unique ? palette[off] : 0u);
+      ++off;
     }
-    __syncthreads();
-  }
+  if (tile == ntiles - 1 && tid == 0 && s_before + total != n_unique) atomicOr(err, kDecBadUnique);
 }
 
-// One pointer-jumping round: (ptr_in, val_in) -> (ptr_out, val_out).
-__global__ void __launch_bounds__(256) decode_jump_kernel(const int32_t *__restrict__ ptr_in,
-                                                          const uint32_t *__restrict__ val_in, int nblk,
-                                                          int32_t *__restrict__ ptr_out,
-                                                          uint32_t *__restrict__ val_out) {
+// Second kernel: each block follows its link to a word and writes its DXT1
+// block. A link leads to an earlier block, so the walk ends; on the way a block
+// replaces its own link (which only it writes) by the one it has just read, so
+// that the blocks behind it skip that part: with all of them walking at once a chain halves
+// at each step, as in pointer jumping, but without a launch and a pass over
+// memory per step (19 launches of 3.7 us before; 3.5 to 9 us now, by the chains). The scan's state is left
+// zeroed for the next frame.
+__global__ void __launch_bounds__(256) decode_link_kernel(const uint8_t *__restrict__ planes, int nblk, uint64_t *link,
+                                                          uint64_t *__restrict__ state, int ntiles,
+                                                          uint32_t *__restrict__ claim, uint64_t *__restrict__ out) {
+  depend();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < ntiles) state[i] = 0ull;
+  if (i == 0) *claim = 0u;
   if (i >= nblk) return;
-  const int32_t p = ptr_in[i];
-  if (p < 0) {
-    ptr_out[i] = -1;
-    val_out[i] = val_in[i];
-    return;
+  uint64_t w = ld_relaxed(link + i);
+  uint8_t v[6];
+#pragma unroll
+  for (int p = 0; p < 6; ++p) v[p] = planes[(size_t)p * nblk + i];
+  while (w < kLinkWord) {
+    w = ld_relaxed(link + w);
+    st_relaxed(link + i, w);
   }
-  const int32_t q = ptr_in[p];
-  if (q < 0) {
-    ptr_out[i] = -1;
-    val_out[i] = val_in[p];
-  } else {
-    ptr_out[i] = q;
-    val_out[i] = 0;
-  }
-}
-
-__global__ void __launch_bounds__(256) decode_assemble_kernel(const uint16_t *__restrict__ ep, const uint32_t *__restrict__ val,
-                                                              int nblk, uint64_t *__restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nblk) return;
-  out[i] = (uint64_t)ep[i] | ((uint64_t)ep[nblk + i] << 16) | ((uint64_t)val[i] << 32);
+  out[i] = (uint64_t)endpoint_word(v[0], v[1], v[2]) | ((uint64_t)endpoint_word(v[3], v[4], v[5]) << 16) | (w << 32);
 }
 
 }  // namespace mptc

@@ -13,6 +13,7 @@
 
 #include "../../include/mptc_gb300.h"
 #include "dxt1_encode.cuh"
+#include "launch.cuh"
 #include "search.cuh"
 #include "learned_search.cuh"
 #include "learned_dict.cuh"
@@ -291,25 +292,6 @@ __global__ void alu_probe_kernel(int iters, int32_t *sink) {
 
 namespace {
 
-// Launches a kernel that calls depend() behind the kernel before it in the stream
-// (programmatic dependent launch). Used inside a frame's chain of kernels, not
-// behind an event wait. A frame is a chain of some 13 kernels of 3 to 20 us; launched
-// this way, with the work area zeroed by the first of them instead of two memsets, an
-// inter frame takes 212 us at 1080p (245 before) and 74.5 us at 256x256 (107).
-template <typename... Par, typename... Arg>
-void launch_chain(void (*kernel)(Par...), int grid, int threads, cudaStream_t s, Arg... arg) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, Par(arg)...);
-}
-
 // The intra pass of an inter frame: fixed-point sweeps over the open blocks,
 // then the exact dataflow kernel only if the sweeps did not converge.
 // Sweeps to run for a configuration's intra_sweeps value.
@@ -324,16 +306,16 @@ int launch_intra_sweeps(const mptc::SearchParams &P, const uint32_t *pending, co
                         uint32_t *sweep, int n, int grid, int sweeps, mptc::SweepPartial *part, int part_cap,
                         cudaStream_t s) {
   if (sweeps == 0) {
-    launch_chain(mptc::intra_search_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, -1, nullptr);
+    mptc::launch_chain(mptc::intra_search_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, -1, nullptr);
     return 1;
   }
   // three estimate buffers: sweep k reads E[k % 3] and, for its skip test,
   // E[(k + 2) % 3] (the estimates sweep k-1 read), and writes E[(k + 1) % 3]
   uint32_t *est[3] = {sweep, sweep + n, sweep + 2 * (size_t)n}, *changed = sweep + 3 * (size_t)n;
   for (int k = 0; k < sweeps; ++k)
-    launch_chain(mptc::intra_sweep_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, est[k % 3],
+    mptc::launch_chain(mptc::intra_sweep_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, est[k % 3],
                  est[(k + 2) % 3], est[(k + 1) % 3], changed + k, changed + k + 1, part, part_cap, k == 0);
-  launch_chain(mptc::intra_search_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, -1,
+  mptc::launch_chain(mptc::intra_search_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, -1,
                changed + sweeps);
   return sweeps + 1;
 }
@@ -354,7 +336,7 @@ int launch_begin(const mptc::SearchParams &P, float4 *wdesc, int ntiles, bool ch
   const uint64_t *words = P.prev ? P.prev : P.stb;
   uint64_t *zeroed = P.prev ? nullptr : P.done;
   if (chained)
-    launch_chain(mptc::weight_desc_kernel, grid, 256, s, words, nblk, wdesc, P.work, n_work, zeroed);
+    mptc::launch_chain(mptc::weight_desc_kernel, grid, 256, s, words, nblk, wdesc, P.work, n_work, zeroed);
   else
     mptc::weight_desc_kernel<<<grid, 256, 0, s>>>(words, nblk, wdesc, P.work, n_work, zeroed);
   return 1;
@@ -403,9 +385,9 @@ int launch_inter_search(const mptc::SearchParams &P, int warps, uint32_t *work, 
   const int nblk = P.bw * P.bh;
   if (P.sa > 8) {
     if (warps == 2)
-      launch_chain(mptc::inter_dedup_kernel<2>, (nblk + 1) / 2, 2 * 32, s, P);
+      mptc::launch_chain(mptc::inter_dedup_kernel<2>, (nblk + 1) / 2, 2 * 32, s, P);
     else
-      launch_chain(mptc::inter_dedup_kernel<4>, (nblk + 3) / 4, 4 * 32, s, P);
+      mptc::launch_chain(mptc::inter_dedup_kernel<4>, (nblk + 3) / 4, 4 * 32, s, P);
     return 1;
   }
   // runs of kInterRun blocks, in a small frame short enough to give every warp
@@ -419,15 +401,15 @@ int launch_inter_search(const mptc::SearchParams &P, int warps, uint32_t *work, 
   uint32_t *next = work + 7, *novf = work + 8;
   // the default search area 8 with its window constants folded
   if (P.sa == 8 && warps == 2)
-    launch_chain(mptc::inter_run_kernel<2, mptc::kRun, 8>, ctas, 2 * 32, s, P, next, run, novf, ovf_list);
+    mptc::launch_chain(mptc::inter_run_kernel<2, mptc::kRun, 8>, ctas, 2 * 32, s, P, next, run, novf, ovf_list);
   else if (P.sa == 8)
-    launch_chain(mptc::inter_run_kernel<4, mptc::kRun, 8>, ctas, 4 * 32, s, P, next, run, novf, ovf_list);
+    mptc::launch_chain(mptc::inter_run_kernel<4, mptc::kRun, 8>, ctas, 4 * 32, s, P, next, run, novf, ovf_list);
   else if (warps == 2)
-    launch_chain(mptc::inter_run_kernel<2, mptc::kRun, 0>, ctas, 2 * 32, s, P, next, run, novf, ovf_list);
+    mptc::launch_chain(mptc::inter_run_kernel<2, mptc::kRun, 0>, ctas, 2 * 32, s, P, next, run, novf, ovf_list);
   else
-    launch_chain(mptc::inter_run_kernel<4, mptc::kRun, 0>, ctas, 4 * 32, s, P, next, run, novf, ovf_list);
+    mptc::launch_chain(mptc::inter_run_kernel<4, mptc::kRun, 0>, ctas, 4 * 32, s, P, next, run, novf, ovf_list);
   // the overflow list is short: four CTAs per SM, idle ones return at once
-  launch_chain(mptc::inter_overflow_kernel<256>, std::min(4 * sm_count, nblk), 256, s, P, ovf_list, novf);
+  mptc::launch_chain(mptc::inter_overflow_kernel<256>, std::min(4 * sm_count, nblk), 256, s, P, ovf_list, novf);
   return 2;
 }
 
@@ -668,7 +650,7 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
                                                            ctx->tile_state, ctx->work + 10, ctx->pending,
                                                            ctx->work + 5, ctx->sweep, changed, flags, ctx->work + 1);
     else
-      launch_chain(mptc::pending_scan_kernel, ctx->ntiles, 256, s, ctx->order, ctx->done, P.stb, ctx->nblk,
+      mptc::launch_chain(mptc::pending_scan_kernel, ctx->ntiles, 256, s, ctx->order, ctx->done, P.stb, ctx->nblk,
                    ctx->ntiles, ctx->tile_state, ctx->work + 10, ctx->pending, ctx->work + 5, ctx->sweep, changed,
                    flags, ctx->work + 1);
   }
@@ -688,7 +670,7 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
   const uint16_t *m16 = P.motion;
   {
     KernelTimer t(ctx, K_UNIQUE, s);
-    launch_chain(mptc::unique_scan_kernel, ctx->ntiles, 256, s, m16, P.stb, ctx->nblk, ctx->ntiles,
+    mptc::launch_chain(mptc::unique_scan_kernel, ctx->ntiles, 256, s, m16, P.stb, ctx->nblk, ctx->ntiles,
                  ctx->tile_state + ctx->ntiles, ctx->work + 11, unique_dev, n_unique_dev, ctx->work + 2,
                  ctx->work + 1);
     ++ctx->launches;
@@ -1097,7 +1079,7 @@ static mptc_status encode_stream_host_run(mptc_ctx *ctx, const uint8_t *frames_h
       st = run_inter_frame(ctx, n_inter++, r.rgb[i], r.up[i], prev, r.fin[i], r.motion[i], r.unique[i],
                            r.n_unique[i], s);
     if (st != MPTC_OK) return lane ? fail(ctx, st, std::string("intra lane: ") + b->err) : st;
-    launch_chain(status_or_kernel, 1, 32, es, lane ? b->work : ctx->work, ctx->run_status);
+    mptc::launch_chain(status_or_kernel, 1, 32, es, lane ? b->work : ctx->work, ctx->run_status);
     ++ctx->launches;
     MPTC_CUDA(cudaEventRecord(r.enc[i], es));
     prev_in_lane = lane;
@@ -1160,7 +1142,7 @@ static mptc_status encode_stream_device_run(mptc_ctx *ctx, const uint8_t *frames
       st = mptc_encode_frame(b, in, nullptr, nullptr, fin, motion_dev + 2 * k * n, unique_dev + k * n,
                              n_unique_dev + k, ctx->lane_s);
       if (st != MPTC_OK) return fail(ctx, st, std::string("intra lane: ") + b->err);
-      launch_chain(status_or_kernel, 1, 32, ctx->lane_s, b->work, ctx->run_status);
+      mptc::launch_chain(status_or_kernel, 1, 32, ctx->lane_s, b->work, ctx->run_status);
       ++ctx->launches;
       MPTC_CUDA(cudaEventRecord(ctx->lane_done, ctx->lane_s));
       prev_in_lane = true;
@@ -1174,7 +1156,7 @@ static mptc_status encode_stream_device_run(mptc_ctx *ctx, const uint8_t *frames
         st = run_inter_frame(ctx, n_inter++, in, nullptr, prev, fin, motion_dev + 2 * k * n, unique_dev + k * n,
                              n_unique_dev + k, s);
       if (st != MPTC_OK) return st;
-      launch_chain(status_or_kernel, 1, 32, s, ctx->work, ctx->run_status);
+      mptc::launch_chain(status_or_kernel, 1, 32, s, ctx->work, ctx->run_status);
       ++ctx->launches;
     }
     prev = fin;
@@ -1510,14 +1492,14 @@ extern "C" mptc_status mptc_encode_frame_noalloc(const mptc_config *cfg, int32_t
   if (prev_final_dev) {
     launch_inter_search(P, kSearchWarps, work, pend, d->sm_count, s);
     const int sw = sweep_count(cfg->intra_sweeps);
-    launch_chain(mptc::pending_scan_kernel, ntiles, 256, s, order, done, stb, n, ntiles, tile_state, work + 10, pend,
+    mptc::launch_chain(mptc::pending_scan_kernel, ntiles, 256, s, order, done, stb, n, ntiles, tile_state, work + 10, pend,
                  work + 5, sweep, sweep + 3 * (size_t)n, sw ? sw + 1 : 0, work + 1);
     launch_intra_sweeps(P, pend, work + 5, sweep, n, d->intra_grid, sw, sweep_part, kSweepPartCapNoalloc, s);
   } else {
     launch_intra_frame(P, order, d->intra_grid, d->sm_count, s);
   }
   const uint16_t *m16 = reinterpret_cast<const uint16_t *>(motion_dev);
-  launch_chain(mptc::unique_scan_kernel, ntiles, 256, s, m16, stb, n, ntiles, tile_state + ntiles, work + 11,
+  mptc::launch_chain(mptc::unique_scan_kernel, ntiles, 256, s, m16, stb, n, ntiles, tile_state + ntiles, work + 11,
                unique_dev, n_unique_dev, work + 2, work + 1);
   noalloc_status_kernel<<<1, 32, 0, s>>>(work, n_unique_dev);
   return cudaGetLastError() == cudaSuccess ? MPTC_OK : MPTC_ECUDA;
@@ -1689,7 +1671,7 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
       mptc_status st = mptc_encode_frame(c->lane_b, frames[i] + k * n * 48, nullptr, nullptr, fin[i] + k * n,
                                          mot[i] + 2 * k * n, uni[i] + k * n, n_uni[i] + k, c->lane_s);
       if (st != MPTC_OK) return st;
-      launch_chain(status_or_kernel, 1, 32, c->lane_s, c->lane_b->work, b->run_status);
+      mptc::launch_chain(status_or_kernel, 1, 32, c->lane_s, c->lane_b->work, b->run_status);
       if (cudaEventRecord(b->lane_ev[i][k], c->lane_s) != cudaSuccess) return MPTC_ECUDA;
     }
   }
@@ -1753,7 +1735,7 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
       if (c->model && !jobs.empty() && cudaStreamWaitEvent(si, b->learned_ev, 0) != cudaSuccess) return MPTC_ECUDA;
       mptc_status st = reencode_finish(c, P[i], uni[i] + k * n, n_uni[i] + k, si);
       if (st != MPTC_OK) return st;
-      launch_chain(status_or_kernel, 1, 32, si, c->work, b->run_status);
+      mptc::launch_chain(status_or_kernel, 1, 32, si, c->work, b->run_status);
       if (cudaEventRecord(c->stb_free[slot[i]], si) != cudaSuccess) return MPTC_ECUDA;
     }
   }

@@ -6,6 +6,7 @@
 
 #include "../../include/mptc_gb300.h"
 #include "endpoint_codec.cuh"
+#include "launch.cuh"
 
 namespace {
 
@@ -17,12 +18,11 @@ bool tiled_size(int32_t width, int32_t height) {
 }  // namespace
 
 struct mptc_decoder {
-  int width = 0, height = 0, bw = 0, bh = 0, nblk = 0, sa = 0, ntiles = 0, rounds = 0;
-  int32_t *ptr[2] = {nullptr, nullptr};
-  uint32_t *val[2] = {nullptr, nullptr};
-  uint32_t *tile_counts = nullptr;
-  uint16_t *ep = nullptr;    // [2][nblk] decoded endpoint words
-  uint32_t *flags = nullptr; // device error flags
+  int width = 0, height = 0, bw = 0, bh = 0, nblk = 0, sa = 0, ntiles = 0;
+  uint64_t *link = nullptr;   // [nblk] index words and copies
+  uint64_t *state = nullptr;  // [ntiles] of the unique blocks' scan, zero between frames; then its tile counter
+  uint8_t *planes = nullptr;  // [6][nblk] decoded endpoint planes
+  uint32_t *flags = nullptr;  // device error flags, status bits
   std::string err;
 };
 
@@ -34,12 +34,9 @@ mptc_status dfail(mptc_decoder *d, mptc_status st, const std::string &msg) {
 }
 
 void release(mptc_decoder *d) {
-  cudaFree(d->ptr[0]);
-  cudaFree(d->ptr[1]);
-  cudaFree(d->val[0]);
-  cudaFree(d->val[1]);
-  cudaFree(d->tile_counts);
-  cudaFree(d->ep);
+  cudaFree(d->link);
+  cudaFree(d->state);
+  cudaFree(d->planes);
   cudaFree(d->flags);
 }
 
@@ -52,8 +49,8 @@ mptc_status mptc_endpoint_coefficients(int32_t width, int32_t height, const uint
   if (!tiled_size(width, height) || !blocks_dev || !coeff_dev) return MPTC_EINVAL;
   const int bw = width / 4, bh = height / 4;
   const dim3 grid(bw / mptc::kTile, bh / mptc::kTile, 6);
-  mptc::endpoint_forward_kernel<<<grid, mptc::kCodecThreads, 0, (cudaStream_t)stream>>>(blocks_dev, bw, bh,
-                                                                                        coeff_dev);
+  mptc::launch_after(mptc::endpoint_forward_kernel, grid, mptc::kCodecThreads, (cudaStream_t)stream, blocks_dev, bw, bh,
+                     coeff_dev);
   return cudaGetLastError() == cudaSuccess ? MPTC_OK : MPTC_ECUDA;
 }
 
@@ -67,20 +64,15 @@ mptc_status mptc_decoder_create(int32_t width, int32_t height, int32_t search_ar
   d->bh = height / 4;
   d->nblk = d->bw * d->bh;
   d->sa = search_area;
-  d->ntiles = (d->nblk + mptc::kDecTile - 1) / mptc::kDecTile;
-  int r = 1;
-  while ((1ll << (r - 1)) < d->nblk) ++r;  // chains are shorter than nblk <= 2^(r-1)
-  d->rounds = r;
+  d->ntiles = (d->nblk + mptc::kScanTile - 1) / mptc::kScanTile;
   const size_t n = (size_t)d->nblk;
-  cudaError_t e = cudaSuccess;
-  for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
-    e = cudaMalloc(&d->ptr[k], n * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&d->val[k], n * sizeof(uint32_t));
-  }
-  if (e == cudaSuccess) e = cudaMalloc(&d->tile_counts, (size_t)d->ntiles * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&d->ep, 2 * n * sizeof(uint16_t));
-  if (e == cudaSuccess) e = cudaMalloc(&d->flags, sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMemset(d->flags, 0, sizeof(uint32_t));
+  const size_t state_bytes = ((size_t)d->ntiles + 1) * sizeof(uint64_t);
+  cudaError_t e = cudaMalloc(&d->link, n * sizeof(uint64_t));
+  if (e == cudaSuccess) e = cudaMalloc(&d->state, state_bytes);
+  if (e == cudaSuccess) e = cudaMemset(d->state, 0, state_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&d->planes, 6 * n);
+  if (e == cudaSuccess) e = cudaMalloc(&d->flags, 2 * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMemset(d->flags, 0, 2 * sizeof(uint32_t));
   if (e != cudaSuccess) {
     release(d);
     delete d;
@@ -105,29 +97,27 @@ mptc_status mptc_decode_frame(mptc_decoder *d, const uint8_t *coeff_dev, const u
     return dfail(d, MPTC_EINVAL, "decode_frame: NULL buffer");
   if (n_unique > (uint32_t)d->nblk) return dfail(d, MPTC_EINVAL, "decode_frame: more unique entries than blocks");
   cudaStream_t s = (cudaStream_t)stream;
-  const dim3 tiles(d->bw / mptc::kTile, d->bh / mptc::kTile, 2);
-  mptc::endpoint_inverse_kernel<<<tiles, mptc::kCodecThreads, 0, s>>>(coeff_dev, d->bw, d->bh, d->ep);
-  mptc::decode_classify_kernel<<<d->ntiles, 256, 0, s>>>(motion_dev, prev_dev, d->bw, d->nblk, d->sa, d->ptr[0],
-                                                         d->val[0], d->tile_counts, d->flags);
-  mptc::decode_unique_kernel<<<d->ntiles, 256, 0, s>>>(motion_dev, d->nblk, d->tile_counts, unique_dev, n_unique,
-                                                       d->val[0], d->flags);
-  const int g = (d->nblk + 255) / 256;
-  int cur = 0;
-  for (int r = 0; r < d->rounds; ++r, cur ^= 1)
-    mptc::decode_jump_kernel<<<g, 256, 0, s>>>(d->ptr[cur], d->val[cur], d->nblk, d->ptr[cur ^ 1], d->val[cur ^ 1]);
-  mptc::decode_assemble_kernel<<<g, 256, 0, s>>>(d->ep, d->val[cur], d->nblk, out_dev);
+  const int tiles = (d->bw / mptc::kTile) * (d->bh / mptc::kTile);
+  uint32_t *claim = reinterpret_cast<uint32_t *>(d->state + d->ntiles);
+  mptc::launch_after(mptc::decode_parts_kernel, d->ntiles + 6 * tiles, mptc::kCodecThreads, s, coeff_dev, d->bw, d->bh,
+                     d->planes, motion_dev, prev_dev, d->sa, unique_dev, n_unique, d->ntiles, d->state, claim, d->link,
+                     d->flags, d->flags + 1);
+  mptc::launch_chain(mptc::decode_link_kernel, (d->nblk + 255) / 256, 256, s, d->planes, d->nblk, d->link, d->state,
+                     d->ntiles, claim, out_dev);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MPTC_OK : dfail(d, MPTC_ECUDA, cudaGetErrorString(e));
 }
 
 mptc_status mptc_decoder_check(mptc_decoder *d, void *stream, uint32_t *flags) {
   if (!d) return MPTC_EINVAL;
-  uint32_t h = 0;
-  cudaError_t e = cudaMemcpyAsync(&h, d->flags, sizeof(h), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d->flags, 0, sizeof(uint32_t), (cudaStream_t)stream);
+  uint32_t w[2] = {0, 0};
+  cudaError_t e = cudaMemcpyAsync(w, d->flags, sizeof(w), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d->flags, 0, sizeof(w), (cudaStream_t)stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
   if (e != cudaSuccess) return dfail(d, MPTC_ECUDA, cudaGetErrorString(e));
+  const uint32_t h = w[0];
   if (flags) *flags = h;
+  if (w[1] & mptc::kDevTimeout) return dfail(d, MPTC_ETIMEOUT, "device-side dependency wait expired");
   if (h) {
     std::string m = "decoded frames held";
     if (h & mptc::kDecBadRef) m += " motion codes that copy from outside the frame or from undecoded blocks";
