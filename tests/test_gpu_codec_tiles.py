@@ -176,3 +176,30 @@ def test_decoder_frames(torch_cuda, w, h, sa, offset):
             prev = words
     finally:
         dec.close()
+
+
+@pytest.mark.parametrize("form", ["strided", "wider", "cpu", "numpy"])
+def test_decoder_input_forms(torch_cuda, form):
+    """Inputs that are not plain CUDA byte tensors are staged: the same blocks."""
+    from mptc_gb300.decoder import Decoder
+    torch = torch_cuda
+    rng = np.random.default_rng(5)
+    n, sa = 64 * 64, 8
+    coeff = rng.integers(0, 256, 6 * n, dtype=np.uint8)
+    motion = codes(rng, "mixed", 64, 64, sa, True).reshape(-1)
+    palette = rng.integers(0, 1 << 32, int((motion.reshape(-1, 2) == 255).all(1).sum()), dtype=np.uint32)
+    t = [torch.from_numpy(a.copy()) for a in (motion, coeff, palette.view(np.int32))]
+    dec = Decoder(256, 256, sa)
+    try:
+        want = dec.decode_frame(*[x.cuda() for x in t]).cpu()
+        if form == "strided":
+            args = [x.cuda().repeat_interleave(2)[::2] for x in t]
+        elif form == "wider":
+            args = [t[0].cuda().to(torch.int32), t[1].cuda().to(torch.int64), t[2].cuda()]
+        else:
+            args = t if form == "cpu" else [motion, coeff, palette]
+        assert torch.equal(dec.decode_frame(*args).cpu(), want)
+        with pytest.raises(RuntimeError):
+            dec.decode_frame(t[0].cuda().view(-1, 2), t[1].cuda(), t[2].cuda())
+    finally:
+        dec.close()
