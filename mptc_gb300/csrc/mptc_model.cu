@@ -15,6 +15,7 @@
 #include "../../include/mptc_gb300.h"
 #include <mutex>
 
+#include "launch.cuh"
 #include "learned.cuh"
 #include "learned_embed.cuh"
 #include "model_internal.h"
@@ -70,16 +71,16 @@ struct mptc_model {
   bf16 *x = nullptr, *h1b = nullptr, *h2b = nullptr, *xc = nullptr, *g1b = nullptr;
   float *f = nullptr, *gg = nullptr;
   bf16 *dfb = nullptr, *dggb = nullptr, *dh1b = nullptr, *dh2b = nullptr, *dg1b = nullptr;
-  float *part = nullptr;  // partial sums of the split gradient reductions (part_floats)
-  size_t part_floats = 0;
-  float *loss = nullptr;
+  float *part = nullptr;        // partial sums of a step's split gradient reductions (part_floats)
+  cudaStream_t side = nullptr;  // the block MLP's stream during a step, forked from and joined to the caller's
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  float *loss = nullptr;  // the loss, then the training kernels' timeout flag (sticky until a step reads it back)
   // packed bf16 weight image of the inference kernels (refreshed after every
   // parameter change) and a bf16 staging buffer for mptc_model_embed
   uint8_t *img = nullptr;
   __nv_bfloat16 *emb_tmp = nullptr;
   int emb_cap = 0;
-  // status words: 0 - 3 of mptc_model_embed; 4 the training kernels' timeout
-  // flag (sticky until a step reads it back)
+  // status words of mptc_model_embed
   uint32_t *status = nullptr;
 };
 
@@ -93,22 +94,37 @@ void free_ws(mptc_model *m) {
   m->dfb = m->dggb = m->dh1b = m->dh2b = m->dg1b = nullptr;
   m->part = nullptr;
   m->cap_b = m->cap_bc = 0;
-  m->part_floats = 0;
 }
 
-// Partial sums of the split dW reductions below (slices x outputs floats).
+// Partial sums of one split dW reduction (slices x outputs floats) at most.
 constexpr size_t kSplitFloats = 1 << 22;
-// Column partial sums of the bias gradients: softmax_ce (2 x 64 per 8
-// blocks) and the dx epilogues (one row of K_layer per 128 examples).
+
+// The split training products run as up to 3 CTAs per SM of a 152-SM part
+// (what two pipeline stages of shared memory allow), fixed so that the
+// split and with it the summation order do not depend on the device.
+constexpr int kTrainCtas = 456;
+
+// Slices of dW[K x N]'s reduction over M examples: of at least 128 rows.
+int dw_splits(int M, int K, int N) {
+  const int tiles = ((N + 127) / 128) * ((K + mptc::kTcBM - 1) / mptc::kTcBM);
+  const int splits = std::min(M / 128, std::max(1, kTrainCtas / tiles));
+  return (int)std::max<size_t>(1, std::min<size_t>((size_t)splits, kSplitFloats / ((size_t)K * N)));
+}
+
+// A step's partial sums: those of the five dW, the column sums of softmax_ce (2
+// x 64 per 8 blocks) and of the dx epilogues (one row per 128 examples).
 size_t part_floats_for(int B, int BC) {
   using namespace mptc;
-  const size_t ce = 2 * (size_t)((B + 7) / 8) * kEmb;
-  const size_t dxb = (size_t)((B + kTcBM - 1) / kTcBM) * kH2;
-  const size_t dxc = (size_t)((BC + kTcBM - 1) / kTcBM) * kCandH;
-  return std::max(std::max(kSplitFloats, ce), std::max(dxb, dxc));
+  size_t n = 2 * (size_t)((B + 7) / 8) * kEmb;
+  for (int l = 0; l < 5; ++l)
+    n += (size_t)dw_splits(l < 3 ? B : BC, kLayers[l].in, kLayers[l].out) * kLayers[l].in * kLayers[l].out;
+  return n + (size_t)((B + kTcBM - 1) / kTcBM) * (kH1 + kH2) + (size_t)((BC + kTcBM - 1) / kTcBM) * kCandH;
 }
 
 mptc_status ensure_ws(mptc_model *m, int B, int BC) {
+  if (!m->side && cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) != cudaSuccess) return MPTC_ECUDA;
+  for (cudaEvent_t &e : m->ev)
+    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return MPTC_ECUDA;
   if (B <= m->cap_b && BC <= m->cap_bc) return MPTC_OK;
   free_ws(m);
   using namespace mptc;
@@ -125,70 +141,79 @@ mptc_status ensure_ws(mptc_model *m, int B, int BC) {
   }
   m->cap_b = B;
   m->cap_bc = BC;
-  m->part_floats = pf;
   return MPTC_OK;
 }
 
 int blocks_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 4096); }
 
-// The split training products run as up to 3 CTAs per SM of a 152-SM part
-// (the most two pipeline stages of shared memory allow), fixed so that the
-// split and with it the summation order do not depend on the device.
-constexpr int kTrainCtas = 456;
+template <bool TA, bool TB, int BN>
+cudaError_t gemm_attr() {
+  return cudaFuncSetAttribute(mptc::gemm_tc_kernel<TA, TB, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              mptc::tc_smem<BN>(2));
+}
 
 cudaError_t ensure_gemm_attrs() {
   static std::once_flag once;
   static cudaError_t err = cudaSuccess;
   std::call_once(once, [] {
-    err = cudaFuncSetAttribute(mptc::gemm_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               mptc::kTcSmem);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(mptc::gemm_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 mptc::kTcSmem);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(mptc::gemm_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 mptc::kTcSmem);
+    for (cudaError_t e : {gemm_attr<false, false, 64>(), gemm_attr<false, false, 128>(), gemm_attr<true, false, 64>(),
+                          gemm_attr<true, false, 128>(), gemm_attr<false, true, 64>(), gemm_attr<false, true, 128>()})
+      if (err == cudaSuccess) err = e;
   });
   return err;
+}
+
+// C[M x N] (contraction K, `splits` slices) with the epilogue e. Tiles of 64
+// columns where N has no more, or where 128 would leave an SM without a tile.
+template <bool TA, bool TB>
+void gemm(const bf16 *A, int lda, const bf16 *B, int ldb, const mptc::GemmEpi &e, int M, int N, int K, int splits,
+          uint32_t *status, cudaStream_t s) {
+  const int rows = (M + mptc::kTcBM - 1) / mptc::kTcBM, steps = mptc::tc_steps(K, splits);
+  if (N <= 64 || rows * ((N + 127) / 128) * splits < 152)
+    mptc::launch_chain_smem(mptc::gemm_tc_kernel<TA, TB, 64>, dim3((N + 63) / 64, rows, splits), 128,
+                            mptc::tc_smem<64>(steps), s, A, lda, B, ldb, e, M, N, K, status);
+  else
+    mptc::launch_chain_smem(mptc::gemm_tc_kernel<TA, TB, 128>, dim3((N + 127) / 128, rows, splits), 128,
+                            mptc::tc_smem<128>(steps), s, A, lda, B, ldb, e, M, N, K, status);
 }
 
 // y[M x N] = x[M x K] W + b (opt. ReLU) into y (fp32) and/or yb (bf16).
 void gemm_fwd(const bf16 *x, const bf16 *W, const float *b, float *y, bf16 *yb, int M, int K, int N, bool relu,
               uint32_t *status, cudaStream_t s) {
-  dim3 grid((N + mptc::kTcBN - 1) / mptc::kTcBN, (M + mptc::kTcBM - 1) / mptc::kTcBM);
-  const mptc::GemmEpi e{y, yb, N, b, relu ? 1 : 0, nullptr, nullptr};
-  mptc::gemm_tc_kernel<false, false><<<grid, 128, mptc::kTcSmem, s>>>(x, K, W, N, e, M, N, K, status);
+  gemm<false, false>(x, K, W, N, {y, yb, N, b, relu ? 1 : 0, nullptr, nullptr}, M, N, K, 1, status, s);
 }
 
-// out[n] = sum of the `slices` rows of part [slices x n], in order.
-void slice_sum(const float *part, int slices, int n, float *out, cudaStream_t s) {
-  mptc::slice_sum_kernel<<<(n + 31) / 32, 256, 0, s>>>(part, slices, n, out);
-}
+// The reductions that a step's last launch sums, and the partial sums' buffer.
+struct Sums {
+  mptc::SumJobs jobs{};
+  float *part;
+  // slices x n partial sums of out, in their order
+  float *add(int slices, int n, float *out) {
+    mptc::SumJob &j = jobs.job[jobs.n];
+    j = {part, out, slices, n, (n + 31) / 32 + (jobs.n ? jobs.job[jobs.n - 1].end : 0)};
+    ++jobs.n;
+    part += (size_t)slices * n;
+    return const_cast<float *>(j.part);
+  }
+};
 
 // dW[K x N] = x^T[K x M] dy[M x N]: few outputs and a long reduction over the
-// M examples, so the reduction is split into slices of at least 256 rows
-// (up to kTrainCtas CTAs in all) whose partial products are summed in slice
-// order afterwards (deterministic).
-void gemm_dw(const bf16 *x, const bf16 *dy, float *dW, int M, int K, int N, float *part, uint32_t *status,
+// M examples, so the reduction is split into slices whose partial products are
+// summed in slice order afterwards (deterministic).
+void gemm_dw(const bf16 *x, const bf16 *dy, float *dW, int M, int K, int N, Sums &sums, uint32_t *status,
              cudaStream_t s) {
-  const int tiles = ((N + mptc::kTcBN - 1) / mptc::kTcBN) * ((K + mptc::kTcBM - 1) / mptc::kTcBM);
-  int splits = std::min(M / 256, std::max(1, kTrainCtas / tiles));
-  splits = (int)std::max<size_t>(1, std::min<size_t>((size_t)splits, kSplitFloats / ((size_t)K * N)));
-  dim3 grid((N + mptc::kTcBN - 1) / mptc::kTcBN, (K + mptc::kTcBM - 1) / mptc::kTcBM, splits);
-  const mptc::GemmEpi e{splits > 1 ? part : dW, nullptr, N, nullptr, 0, nullptr, nullptr};
-  mptc::gemm_tc_kernel<true, false><<<grid, 128, mptc::kTcSmem, s>>>(x, K, dy, N, e, K, N, M, status);
-  if (splits > 1) slice_sum(part, splits, K * N, dW, s);
+  const int splits = dw_splits(M, K, N);
+  float *C = splits > 1 ? sums.add(splits, K * N, dW) : dW;
+  gemm<true, false>(x, K, dy, N, {C, nullptr, N, nullptr, 0, nullptr, nullptr}, K, N, M, splits, status, s);
 }
 
 // dx[M x K] = (dy[M x N] W^T) masked by the ReLU of the layer's input (h > 0)
-// into dxb (bf16), and db[K] = the column sums of that dx (the bias gradient
-// of the layer below).
-void gemm_dx(const bf16 *dy, const bf16 *W, const bf16 *h, bf16 *dxb, float *db, int M, int K, int N, float *part,
+// into dxb (bf16), and the partial column sums of that dx, whose total is db[K]
+// (the bias gradient of the layer below).
+void gemm_dx(const bf16 *dy, const bf16 *W, const bf16 *h, bf16 *dxb, float *db, int M, int K, int N, Sums &sums,
              uint32_t *status, cudaStream_t s) {
-  dim3 grid((K + mptc::kTcBN - 1) / mptc::kTcBN, (M + mptc::kTcBM - 1) / mptc::kTcBM);
-  const mptc::GemmEpi e{nullptr, dxb, K, nullptr, 0, h, part};
-  mptc::gemm_tc_kernel<false, true><<<grid, 128, mptc::kTcSmem, s>>>(dy, N, W, N, e, M, K, N, status);
-  slice_sum(part, (int)grid.y, K, db, s);
+  float *part = sums.add((M + mptc::kTcBM - 1) / mptc::kTcBM, K, db);
+  gemm<false, true>(dy, N, W, N, {nullptr, dxb, K, nullptr, 0, h, part}, M, K, N, 1, status, s);
 }
 
 // Forward through both MLPs for a training batch; then, if `grads`, the loss
@@ -206,50 +231,65 @@ mptc_status forward_backward(mptc_model *m, const uint8_t *rgb, int width, int b
     b[l] = m->w + kOff.b[l];
   }
   if (ensure_gemm_attrs() != cudaSuccess) return MPTC_ECUDA;
-  uint32_t *status = m->status + 4;
-  block_features_kernel<<<blocks_for((size_t)B * kFeatPad), 256, 0, s>>>(rgb, width, bw, stb, blocks, B, m->x);
-  gemm_fwd(m->x, W[0], b[0], nullptr, m->h1b, B, kFeatPad, kH1, true, status, s);
-  gemm_fwd(m->h1b, W[1], b[1], nullptr, m->h2b, B, kH1, kH2, true, status, s);
-  gemm_fwd(m->h2b, W[2], b[2], m->f, nullptr, B, kH2, kEmb, false, status, s);
-  cand_features_kernel<<<blocks_for((size_t)BC * kCandIn), 256, 0, s>>>(cands, 1, BC, m->xc);
+  uint32_t *status = reinterpret_cast<uint32_t *>(m->loss + 1);
+  // The block MLP runs on the side stream beside the candidate MLP, forward and
+  // backward: its products are a few tiles each (4096 rows: 64 CTAs), a chain of
+  // launches whose latencies the candidates' products cover.
+  cudaStream_t t = m->side;
+  cudaMemsetAsync(m->loss, 0, sizeof(float), s);
+  bool ok = cudaEventRecord(m->ev[0], s) == cudaSuccess && cudaStreamWaitEvent(t, m->ev[0], 0) == cudaSuccess;
+  if (!ok) return MPTC_ECUDA;
+  block_features_kernel<<<blocks_for((size_t)B * 2), 256, 0, t>>>(rgb, width, bw, stb, blocks, B, m->x);
+  gemm_fwd(m->x, W[0], b[0], nullptr, m->h1b, B, kFeatPad, kH1, true, status, t);
+  gemm_fwd(m->h1b, W[1], b[1], nullptr, m->h2b, B, kH1, kH2, true, status, t);
+  gemm_fwd(m->h2b, W[2], b[2], m->f, nullptr, B, kH2, kEmb, false, status, t);
+  ok = cudaEventRecord(m->ev[1], t) == cudaSuccess;
+  cand_features_kernel<<<blocks_for((size_t)BC * kCandIn / 8), 256, 0, s>>>(cands, 1, BC, m->xc);
   gemm_fwd(m->xc, W[3], b[3], nullptr, m->g1b, BC, kCandIn, kCandH, true, status, s);
   gemm_fwd(m->g1b, W[4], b[4], m->gg, nullptr, BC, kCandH, kEmb, false, status, s);
-  cudaMemsetAsync(m->loss, 0, sizeof(float), s);
-  const int nce = (B + 7) / 8;
-  float *partF = m->part, *partG = m->part + (size_t)nce * kEmb;
-  softmax_ce_kernel<<<nce, 256, 0, s>>>(m->f, m->gg, B, C, m->dfb, m->dggb, partF, partG, m->loss);
-  if (!grads) return cudaGetLastError() == cudaSuccess ? MPTC_OK : MPTC_ECUDA;
+  ok = cudaStreamWaitEvent(s, m->ev[1], 0) == cudaSuccess && ok;
   float *G[5], *Gb[5];
   for (int l = 0; l < 5; ++l) {
     G[l] = m->g + kOff.w[l];
     Gb[l] = m->g + kOff.b[l];
   }
-  // output biases from the loss kernel's column sums
-  slice_sum(partF, nce, kEmb, Gb[2], s);
-  slice_sum(partG, nce, kEmb, Gb[4], s);
+  const int nce = (B + 7) / 8;
+  Sums sums;
+  sums.part = m->part;
+  float *partF = sums.add(nce, kEmb, Gb[2]), *partG = sums.add(nce, kEmb, Gb[4]);  // the output biases
+  softmax_ce_kernel<<<nce, 256, 0, s>>>(m->f, m->gg, B, C, m->dfb, m->dggb, partF, partG, m->loss);
+  if (!grads) return ok && cudaGetLastError() == cudaSuccess ? MPTC_OK : MPTC_ECUDA;
+  ok = cudaEventRecord(m->ev[0], s) == cudaSuccess && cudaStreamWaitEvent(t, m->ev[0], 0) == cudaSuccess && ok;
+  if (!ok) return MPTC_ECUDA;
   // block MLP
-  gemm_dw(m->h2b, m->dfb, G[2], B, kH2, kEmb, m->part, status, s);
-  gemm_dx(m->dfb, W[2], m->h2b, m->dh2b, Gb[1], B, kH2, kEmb, m->part, status, s);
-  gemm_dw(m->h1b, m->dh2b, G[1], B, kH1, kH2, m->part, status, s);
-  gemm_dx(m->dh2b, W[1], m->h1b, m->dh1b, Gb[0], B, kH1, kH2, m->part, status, s);
-  gemm_dw(m->x, m->dh1b, G[0], B, kFeatPad, kH1, m->part, status, s);
+  gemm_dx(m->dfb, W[2], m->h2b, m->dh2b, Gb[1], B, kH2, kEmb, sums, status, t);
+  gemm_dx(m->dh2b, W[1], m->h1b, m->dh1b, Gb[0], B, kH1, kH2, sums, status, t);
+  gemm_dw(m->h2b, m->dfb, G[2], B, kH2, kEmb, sums, status, t);
+  gemm_dw(m->h1b, m->dh2b, G[1], B, kH1, kH2, sums, status, t);
+  gemm_dw(m->x, m->dh1b, G[0], B, kFeatPad, kH1, sums, status, t);
+  ok = cudaEventRecord(m->ev[1], t) == cudaSuccess;
   // candidate MLP
-  gemm_dw(m->g1b, m->dggb, G[4], BC, kCandH, kEmb, m->part, status, s);
-  gemm_dx(m->dggb, W[4], m->g1b, m->dg1b, Gb[3], BC, kCandH, kEmb, m->part, status, s);
-  gemm_dw(m->xc, m->dg1b, G[3], BC, kCandIn, kCandH, m->part, status, s);
-  return cudaGetLastError() == cudaSuccess ? MPTC_OK : MPTC_ECUDA;
+  gemm_dx(m->dggb, W[4], m->g1b, m->dg1b, Gb[3], BC, kCandH, kEmb, sums, status, s);
+  gemm_dw(m->g1b, m->dggb, G[4], BC, kCandH, kEmb, sums, status, s);
+  gemm_dw(m->xc, m->dg1b, G[3], BC, kCandIn, kCandH, sums, status, s);
+  ok = cudaStreamWaitEvent(s, m->ev[1], 0) == cudaSuccess && ok;
+  slice_sum_kernel<<<sums.jobs.job[sums.jobs.n - 1].end, 32 * kSumWarps, 0, s>>>(sums.jobs);
+  return ok && cudaGetLastError() == cudaSuccess ? MPTC_OK : MPTC_ECUDA;
 }
 
 // Reads back (and clears) the training kernels' timeout flag after the work
 // queued on s, together with the loss when loss_host is given.
 mptc_status finish_training(mptc_model *m, float *loss_host, cudaStream_t s) {
-  uint32_t flag = 0;
-  if ((loss_host && cudaMemcpyAsync(loss_host, m->loss, sizeof(float), cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
-      cudaMemcpyAsync(&flag, m->status + 4, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+  struct {
+    float loss;
+    uint32_t flag;
+  } h;
+  if (cudaMemcpyAsync(&h, m->loss, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return MPTC_ECUDA;
-  if (flag) {
-    cudaMemsetAsync(m->status + 4, 0, 4, s);
+  if (loss_host) *loss_host = h.loss;
+  if (h.flag) {
+    cudaMemsetAsync(m->loss + 1, 0, sizeof(uint32_t), s);
     return MPTC_ETIMEOUT;
   }
   return MPTC_OK;
@@ -356,8 +396,9 @@ mptc_status mptc_model_create(uint64_t seed, mptc_model **out) {
   if (!m) return MPTC_ENOMEM;
   const size_t n = kOff.total;
   if (dmalloc(&m->w, n) || dmalloc(&m->wb, n) || dmalloc(&m->g, n) || dmalloc(&m->m, n) || dmalloc(&m->v, n) ||
-      dmalloc(&m->loss, 1) || dmalloc(&m->img, mptc::kImgBytes) || dmalloc(&m->status, 8) ||
-      cudaMemset(m->img, 0, mptc::kImgBytes) != cudaSuccess || cudaMemset(m->status, 0, 32) != cudaSuccess) {
+      dmalloc(&m->loss, 2) || dmalloc(&m->img, mptc::kImgBytes) || dmalloc(&m->status, 8) ||
+      cudaMemset(m->img, 0, mptc::kImgBytes) != cudaSuccess || cudaMemset(m->status, 0, 32) != cudaSuccess ||
+      cudaMemset(m->loss, 0, 2 * sizeof(float)) != cudaSuccess) {
     mptc_model_destroy(m);
     return MPTC_ENOMEM;
   }
@@ -389,6 +430,9 @@ mptc_status mptc_model_create(uint64_t seed, mptc_model **out) {
 mptc_status mptc_model_destroy(mptc_model *m) {
   if (!m) return MPTC_EINVAL;
   free_ws(m);
+  if (m->side) cudaStreamDestroy(m->side);
+  for (cudaEvent_t e : m->ev)
+    if (e) cudaEventDestroy(e);
   cudaFree(m->w);
   cudaFree(m->wb);
   cudaFree(m->g);
