@@ -1,5 +1,5 @@
-// InterBlockSearch (codec/dxt_image.cpp:715-774): the one-block search, the
-// run search for sa <= 8 and the overflow search of noisy runs.
+// InterBlockSearch (codec/dxt_image.cpp:715-774): the run search for sa <= 8 with
+// the overflow search of noisy runs, and the search of wider windows.
 #pragma once
 #include <cstdint>
 
@@ -11,201 +11,14 @@ namespace mptc {
 // InterBlockSearch, codec/dxt_image.cpp:715-774: rows j = by-sa .. by+sa-1,
 // columns i = bx-sa .. bx+sa-1 (both ascending); motion (i-bx+sa)|0x80,
 // (j-by+sa)|0x80. Accepted blocks become final here; the others are left for
-// the intra pass (done = 0). One warp per block.
+// the intra pass (done = 0).
 // Refit, validity and error depend only on the block and the candidate index
 // word, so positions holding equal words get equal results, and each distinct
 // word of the window is evaluated once: on smooth content a 16x16 window holds
 // few distinct words (about 15% of the positions on the 1080p test stream).
-// Per span of up to 256 positions (the whole window for sa <= 8): the warp
-// loads the candidates, inserts the distinct words other than the block's own
-// into a shared hash table (open addressing with as many buckets as positions,
-// so an insertion always ends; own word = empty marker: the identity
-// candidate needs no refit), evaluates the distinct words 32 at a time and
-// records each position's result in the lane's selection statistics
-// (LaneSel); warp_select then applies the reference's selection rule.
-constexpr int kDedupSpan = 256;     // positions per dedup span (8 chunks)
-constexpr int kDedupBuckets = 256;  // hash buckets (a span has <= 256 distinct words)
-
-struct DedupTab {
-  uint32_t key[kDedupBuckets];  // index word, or the block's own word when empty
-  uint16_t slot[kDedupBuckets];
-  uint32_t nidx[kDedupSpan];    // a window block holding each distinct word
-  uint16_t bkt[kDedupSpan];     // the bucket holding each distinct word
-  int e[kDedupSpan];
-  uint32_t eps[kDedupSpan];
-};
-
-__device__ __forceinline__ uint32_t dedup_hash(uint32_t v) { return (v * 2654435761u) >> 24; }
-
-// The exhaustive inter search of block idx by one warp: every distinct window
-// word evaluated once, the reference's selection, the final block and motion
-// code written when accepted. Returns the block's completion word (0: left
-// open for the intra pass), the same in every lane.
-__device__ __forceinline__ uint64_t inter_block_search(const SearchParams &P, const BlockTab &tab, DedupTab &dd,
-                                                       const PixelGroups &pg, const uint8_t *s_snap5,
-                                                       const uint8_t *s_snap6, int idx, int bx, int by,
-                                                       uint64_t stb, int orig, int sumsq, int lane) {
-  const uint32_t own = (uint32_t)(stb >> 32);
-  const unsigned lt_mask = (1u << lane) - 1u;
-  const int w2 = 2 * P.sa, npos = w2 * w2;
-  // pos / w2 as one multiply-high: exact for pos < 2^16 and w2 <= 126
-  const uint32_t w2_magic = 0xFFFFFFFFu / (uint32_t)w2 + 1u;
-  const uint32_t *prev_hi = reinterpret_cast<const uint32_t *>(P.prev) + 1;
-  LaneSel ls_;
-  int ls[8];  // slot of each of the lane's positions in the current span
-  for (int span = 0; span < npos; span += kDedupSpan) {
-    for (int b = lane; b < kDedupBuckets; b += 32) dd.key[b] = own;
-    __syncwarp();
-    uint32_t lc[8], ln[8];
-    unsigned valid = 0;
-    int nuniq = 0;
-    // all candidate loads of the span first, so their latencies overlap
-    {
-      const int pos0 = span + lane;
-      int row = pos0 / w2, col = pos0 - row * w2;
-      const int drow = 32 / w2, dcol = 32 - drow * w2;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const int pos = pos0 + 32 * c;
-        const int j = by - P.sa + row, i = bx - P.sa + col;
-        uint32_t cand = own, nidx = 0;
-        if (pos < npos && i >= 0 && j >= 0 && i < P.bw && j < P.bh) {
-          nidx = (uint32_t)(j * P.bw + i);
-          cand = __ldg(prev_hi + 2 * (size_t)nidx);
-          valid |= 1u << c;
-        }
-        lc[c] = cand;
-        ln[c] = nidx;
-        row += drow;
-        col += dcol;
-        if (col >= w2) {
-          col -= w2;
-          ++row;
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const uint32_t cand = lc[c], nidx = ln[c];
-      const bool need = cand != own;  // invalid positions hold `own` too
-      const unsigned peers = __match_any_sync(kFull, cand);
-      const int leader = __ffs(peers) - 1;
-      uint32_t b = dedup_hash(cand);
-      bool is_new = false, found = false;
-      if (need && lane == leader) {
-        for (int probe = 0; probe < kDedupBuckets; ++probe) {
-          const uint32_t old = atomicCAS(&dd.key[b], own, cand);
-          if (old == own) {
-            is_new = true;
-            break;
-          }
-          if (old == cand) {
-            found = true;
-            break;
-          }
-          b = (b + 1) & (kDedupBuckets - 1);
-        }
-      }
-      const unsigned newm = __ballot_sync(kFull, is_new);
-      int slot = -1;
-      if (is_new) {
-        slot = nuniq + __popc(newm & lt_mask);
-        dd.slot[b] = (uint16_t)slot;
-        dd.nidx[slot] = nidx;
-        dd.bkt[slot] = (uint16_t)b;
-      } else if (found) {
-        slot = dd.slot[b];  // inserted by an earlier chunk of this span
-      }
-      ls[c] = __shfl_sync(kFull, slot, leader);
-      nuniq += __popc(newm);
-      __syncwarp();  // this chunk's slot writes land before later chunks read them
-    }
-    __syncwarp();
-    for (int k = lane; k < nuniq; k += 32) {
-      const uint32_t nidx = dd.nidx[k], cand = dd.key[dd.bkt[k]];
-      const float4 d = __ldg(P.wdesc + nidx);
-      const WeightSums ws{d.x, d.y, d.z, d.w};
-      uint32_t eps = 0;
-      int refit = 0;
-      dd.e[k] = eval_candidate(tab, pg, s_snap5, s_snap6, cand, ws, own, orig, sumsq, eps, refit);
-      dd.eps[k] = eps;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      if ((valid >> c) & 1u) {
-        const int pos = span + 32 * c + lane;
-        ls_.add(pos, (int)__umulhi((uint32_t)pos, w2_magic), lc[c] == own ? 0 : dd.e[ls[c]]);
-      }
-    }
-    __syncwarp();
-  }
-  int m;
-  const int sel = warp_select(ls_, w2, m);
-  const bool accept = sel >= 0 && m <= P.thr;  // warp-uniform
-  uint64_t word = 0;
-  if (accept) {
-    // the selected position's index word and refit: the owning lane looks
-    // them up (one span; slot -1 marks the block's own word) or evaluates the
-    // word again (several spans)
-    const int owner = sel & 31;
-    uint64_t blk = 0;
-    if (lane == owner) {
-      if (npos <= kDedupSpan) {
-        const int c = sel >> 5;
-        int slot = -1;
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc)
-          if (cc == c) slot = ls[cc];
-        blk = slot < 0 ? stb : ((uint64_t)dd.eps[slot] | ((uint64_t)dd.key[dd.bkt[slot]] << 32));
-      } else {
-        const int i = bx - P.sa + sel % w2, j = by - P.sa + sel / w2;
-        const uint32_t cand = __ldg(prev_hi + 2 * (size_t)(j * P.bw + i));
-        if (cand == own) {
-          blk = stb;
-        } else {
-          const float4 d = __ldg(P.wdesc + (size_t)(j * P.bw + i));
-          const WeightSums ws{d.x, d.y, d.z, d.w};
-          uint32_t eps = 0;
-          int refit = 0;
-          eval_candidate(tab, pg, s_snap5, s_snap6, cand, ws, own, orig, sumsq, eps, refit);
-          blk = (uint64_t)eps | ((uint64_t)cand << 32);
-        }
-      }
-      const int row = sel / w2, col = sel - row * w2;
-      P.final_blk[idx] = blk;
-      P.motion[idx] = (uint16_t)((col | 0x80) | ((row | 0x80) << 8));
-      word = done_word(blk);
-    }
-    word = __shfl_sync(kFull, word, owner);
-  }
-  return word;
-}
-
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) inter_dedup_kernel(SearchParams P) {
-  __shared__ BlockTab s_tab[WARPS];
-  __shared__ DedupTab s_dd[WARPS];
-  __shared__ uint8_t s_snap5[256], s_snap6[256];
-  build_snap_tables(s_snap5, s_snap6);
-  __syncthreads();
-  depend();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  BlockTab &tab = s_tab[warp];
-  const int nblk = P.bw * P.bh;
-  for (int idx = blockIdx.x * WARPS + warp; idx < nblk; idx += gridDim.x * WARPS) {
-    const int by = idx / P.bw, bx = idx - by * P.bw;
-    const int sumsq = stage_block(tab, P.rgb, P.width, bx, by, lane);
-    const PixelGroups pg = load_groups(tab);
-    const uint64_t word = inter_block_search(P, tab, s_dd[warp], pg, s_snap5, s_snap6, idx, bx, by, P.stb[idx],
-                                             P.orig_err[idx], sumsq, lane);
-    if (lane == 0) P.done[idx] = word;
-    __syncwarp();
-  }
-}
 
 // ------------------------------------------------------------ inter runs --
-// The same search for sa <= 8, one warp per run of up to kRun horizontally
+// The search for sa <= 8, one warp per run of up to kRun horizontally
 // adjacent blocks of a row. Their windows share all rows and overlap in all but
 // a few columns, so the warp deduplicates the union of the windows (w2 rows of
 // at most w2 + kRun - 1 columns, a row at a time, lane = column) once, recording
@@ -234,11 +47,13 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) inter_dedup_kernel(Sea
 constexpr int kRun = 8;
 constexpr int kRunWords = 128;  // distinct union words handled by the run table
 constexpr int kRunBuckets = 256;
+__device__ __forceinline__ uint32_t run_hash(uint32_t v) { return (v * 2654435761u) >> 24; }
 // err_diff e as a rank: 0 for e < 0, e + 1 for the others (err_diffs are at most
 // 65025), kNoRank where the refit would swap the endpoints
 constexpr uint32_t kNoRank = 0xFFFFu;
 
 struct RunTab {
+  static constexpr int kSlotBits = 8;  // of a pair's word; its block above them
   static constexpr int kCols = 16 + kRun - 1;  // union columns at sa = 8
   static constexpr int kStride = kCols + 1;
   // the marker, kRunWords words, and the up to kCols further new words of the
@@ -268,9 +83,10 @@ struct RunTab {
 };
 
 // Evaluates a pair of a run from the integer sums; false where run_exact has to.
-__device__ __forceinline__ bool run_quick(const RunTab &rt, const float4 *wdesc, const SnapTables &st, uint32_t pair,
+template <class Tab>
+__device__ __forceinline__ bool run_quick(const Tab &rt, const float4 *wdesc, const SnapTables &st, uint32_t pair,
                                           int &e) {
-  const int k = (int)(pair >> 8), s = (int)(pair & 255u);
+  const int k = (int)(pair >> Tab::kSlotBits), s = (int)(pair & ((1u << Tab::kSlotBits) - 1u));
   const float4 d = __ldg(wdesc + rt.at[s]);
   const WeightSums ws{d.x, d.y, d.z, d.w};
   RefitValues r;
@@ -280,8 +96,9 @@ __device__ __forceinline__ bool run_quick(const RunTab &rt, const float4 *wdesc,
   return ok;
 }
 // Evaluates a pair by the reference's own steps: its err_diff and endpoints.
-__device__ __forceinline__ uint2 run_exact(const RunTab &rt, const float4 *wdesc, const SnapTables &st, uint32_t pair) {
-  const int k = (int)(pair >> 8), s = (int)(pair & 255u);
+template <class Tab>
+__device__ __forceinline__ uint2 run_exact(const Tab &rt, const float4 *wdesc, const SnapTables &st, uint32_t pair) {
+  const int k = (int)(pair >> Tab::kSlotBits), s = (int)(pair & ((1u << Tab::kSlotBits) - 1u));
   const float4 d = __ldg(wdesc + rt.at[s]);
   const WeightSums ws{d.x, d.y, d.z, d.w};
   RefitValues r;
@@ -292,6 +109,28 @@ __device__ __forceinline__ uint2 run_exact(const RunTab &rt, const float4 *wdesc
 }
 __device__ __forceinline__ uint16_t run_rank(int e) {
   return (uint16_t)(e == kInvalid ? kNoRank : (uint32_t)max(e, -1) + 1u);
+}
+
+// The pixels of a run's nb blocks by one warp, one block row per lane.
+__device__ __forceinline__ void stage_run(PixBlock *px, const SearchParams &P, int bx0, int by, int nb, int lane) {
+  const int k = lane >> 2, r = lane & 3;
+  uint32_t c0 = 0, c1 = 0, c2 = 0;
+  if (k < nb) load_channels(P.rgb, P.width, bx0 + k, 4 * by + r, c0, c1, c2);
+  uint32_t s0 = __dp4a(c0, 0x01010101u, 0u), s1 = __dp4a(c1, 0x01010101u, 0u), s2 = __dp4a(c2, 0x01010101u, 0u);
+  uint32_t sq = __dp4a(c0, c0, __dp4a(c1, c1, __dp4a(c2, c2, 0u)));
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    s0 += __shfl_xor_sync(kFull, s0, o);
+    s1 += __shfl_xor_sync(kFull, s1, o);
+    s2 += __shfl_xor_sync(kFull, s2, o);
+    sq += __shfl_xor_sync(kFull, sq, o);
+  }
+  if (k < nb) {
+    px[k].pg[0][r] = c0;
+    px[k].pg[1][r] = c1;
+    px[k].pg[2][r] = c2;
+    if (r == 0) *reinterpret_cast<uint4 *>(px[k].sum) = make_uint4(s0, s1, s2, sq);
+  }
 }
 
 // SA: the search area when fixed at compile time (its constants fold), 0 to
@@ -342,28 +181,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
         }
     }
     __syncwarp();
-    // the blocks' pixels, one block row per lane
-    {
-      const int k = lane >> 2, r = lane & 3;
-      uint32_t c0 = 0, c1 = 0, c2 = 0;
-      if (k < nb) load_channels(P.rgb, P.width, bx0 + k, 4 * by + r, c0, c1, c2);
-      uint32_t s0 = __dp4a(c0, 0x01010101u, 0u), s1 = __dp4a(c1, 0x01010101u, 0u), s2 = __dp4a(c2, 0x01010101u, 0u);
-      uint32_t sq = __dp4a(c0, c0, __dp4a(c1, c1, __dp4a(c2, c2, 0u)));
-#pragma unroll
-      for (int o = 1; o <= 2; o <<= 1) {
-        s0 += __shfl_xor_sync(kFull, s0, o);
-        s1 += __shfl_xor_sync(kFull, s1, o);
-        s2 += __shfl_xor_sync(kFull, s2, o);
-        sq += __shfl_xor_sync(kFull, sq, o);
-      }
-      if (k < nb) {
-        PixBlock &px = rt.px[k];
-        px.pg[0][r] = c0;
-        px.pg[1][r] = c1;
-        px.pg[2][r] = c2;
-        if (r == 0) *reinterpret_cast<uint4 *>(px.sum) = make_uint4(s0, s1, s2, sq);
-      }
-    }
+    stage_run(rt.px, P, bx0, by, nb, lane);
     // the distinct words, row by row: a word's first lane looks it up
     int nuniq = 1;
     uint32_t mark_cols = 0, mark_at = 0;  // the marker's
@@ -382,7 +200,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
           mark_cols |= peers;
           if (peers) mark_at = (uint32_t)(j * P.bw + i0 + __ffs(peers) - 1);
         } else if (lane == __ffs(peers) - 1) {
-          b = dedup_hash(cand);
+          b = run_hash(cand);
           uint32_t old;
           while ((old = atomicCAS(&rt.bkey[b], marker, cand)) != marker && old != cand)
             b = (b + 1) & (kRunBuckets - 1);  // ends: at most kSlots - 1 words in kRunBuckets
@@ -558,6 +376,238 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
       P.done[idx] = word;
     }
     __syncwarp();
+  }
+}
+
+// ------------------------------------------------------------ wide windows --
+// The search for sa > 8, one CTA per run of up to kRun adjacent blocks: the same
+// three parts as a run of inter_run_kernel, over the union of the run's windows,
+// w2 rows of w2 + kRun - 1 columns (up to 126 x 133), by eight warps.
+// 1. Every position's word is looked up in a hash table in shared memory, a
+//    compare-and-swap only where a plain read finds an empty bucket, and the
+//    position keeps the bucket.
+// 2. Every pair of a block and a distinct word is evaluated (words at the
+//    union's edges also for the blocks whose window they miss, which no position
+//    then selects): a warp takes 32 words of one block, refit_quick, the near ties
+//    queued for refit_exact. Results are 16-bit ranks by block and bucket.
+// 3. A warp per block takes the reference's selection over the window's
+//    positions, and one warp refits the selected words for their endpoints.
+// A union of more distinct words than the table takes (noise) is searched in
+// slabs of rows that fit it, whose selections are merged.
+// A warp per block and a table per span of 256 positions before: 510 us for an
+// 856x480 frame at sa 24, under 200 now (the whole frame 302, before 642).
+constexpr int kWideThreads = 256, kWideBuckets = 1024, kWideWords = 640;
+// The buckets' table is never full: a thread inserts only after it has read a
+// count of at most kWideWords, and counts each word before its next.
+static_assert(kWideWords + kWideThreads < kWideBuckets, "a probe ends at an empty bucket");
+static_assert(kWideWords >= 126 + kRun - 1, "a row of any union fits");
+
+struct WideTab {
+  static constexpr int kSlotBits = 11;
+  static constexpr int kMark = kWideBuckets;      // slot of the empty buckets' word, the first block's own
+  static constexpr int kNone = kWideBuckets + 1;  // slot of out-of-frame positions
+  PixBlock px[kRun];
+  int orig[kRun];
+  uint32_t own[kRun];
+  uint32_t key[kWideBuckets + 1];
+  uint32_t at[kWideBuckets + 1];  // a block of the previous frame holding the word
+  uint16_t list[kWideBuckets];    // the used buckets
+  uint16_t rank[kRun][kWideBuckets + 2];
+  uint16_t exact[kWideThreads / 32][64];  // a warp's near ties: block << kSlotBits | slot
+  int win[kRun];                  // selected position (-1: none)
+  int n;                          // used buckets
+};
+// The dynamic shared memory: the table and a 16-bit slot per union position.
+__host__ __device__ constexpr int wide_smem(int sa) {
+  return (int)sizeof(WideTab) + 2 * (2 * sa) * (2 * sa + kRun - 1);
+}
+
+__global__ void __launch_bounds__(kWideThreads, 4) inter_wide_kernel(SearchParams P, int run) {
+  extern __shared__ __align__(16) uint8_t wide_mem[];
+  __shared__ SnapTables s_snap;
+  WideTab &wt = *reinterpret_cast<WideTab *>(wide_mem);
+  uint16_t *pslot = reinterpret_cast<uint16_t *>(wide_mem + sizeof(WideTab));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  constexpr int kWarps = kWideThreads / 32;
+  build_snap_edges(s_snap);
+  depend();
+  const int per_row = (P.bw + run - 1) / run, by = blockIdx.x / per_row;
+  const int bx0 = (blockIdx.x - by * per_row) * run, nb = min(run, P.bw - bx0);
+  const int sa = P.sa, w2 = 2 * sa, cols = w2 + nb - 1, j0 = by - sa, i0 = bx0 - sa;
+  const uint32_t *prev_hi = reinterpret_cast<const uint32_t *>(P.prev) + 1;
+  const uint32_t marker = (uint32_t)(P.stb[by * P.bw + bx0] >> 32);
+  if (warp == 0) {
+    if (lane < nb) {
+      wt.orig[lane] = P.orig_err[by * P.bw + bx0 + lane];
+      wt.own[lane] = (uint32_t)(P.stb[by * P.bw + bx0 + lane] >> 32);
+      wt.rank[lane][WideTab::kNone] = (uint16_t)kNoRank;
+    }
+    stage_run(wt.px, P, bx0, by, nb, lane);
+  }
+  volatile uint32_t *key = wt.key;
+  volatile int *count = &wt.n;
+  // warp k: its block's selection so far (see LaneSel): the smallest rank at its first
+  // position, the first err_diff <= 0, an err_diff < 0 in the last row that holds one
+  uint32_t best = 0xFFFFFFFFu, first = 1u << 14;
+  int last = -1;
+  int slab = w2;  // rows at a time
+  for (int r0 = 0; r0 < w2;) {
+    const int r1 = min(w2, r0 + slab);
+    __syncthreads();  // the previous slab's readers are done
+    for (int b = tid; b <= kWideBuckets; b += kWideThreads) wt.key[b] = marker;
+    if (tid == 0) {
+      wt.n = 0;
+      wt.at[WideTab::kMark] = ~0u;
+    }
+    __syncthreads();
+    // 1. the distinct words
+    for (int r = r0 + warp; r < r1; r += kWarps) {
+      if (__any_sync(kFull, *count > kWideWords)) break;
+      const int j = j0 + r;
+      const bool row_in = j >= 0 && j < P.bh;
+      const uint32_t *src = prev_hi + 2 * ((ptrdiff_t)j * P.bw + i0);
+      auto in = [&](int c) { return row_in && c < cols && i0 + c >= 0 && i0 + c < P.bw; };
+      uint32_t next = in(lane) ? __ldg(src + 2 * lane) : marker;
+#pragma unroll 1
+      for (int c = lane; c < cols + lane; c += 32) {  // the warp's lanes together
+        const uint32_t cand = next;
+        if (in(c + 32)) next = __ldg(src + 2 * (c + 32));
+        if (c >= cols) continue;
+        uint32_t slot = WideTab::kNone;
+        if (in(c)) {
+          const uint32_t nidx = (uint32_t)(j * P.bw + i0 + c);
+          if (cand == marker) {
+            slot = WideTab::kMark;
+            wt.at[WideTab::kMark] = nidx;  // any of them
+          } else {
+            uint32_t b = (cand * 2654435761u) >> 22;
+            for (;;) {
+              uint32_t old = key[b];
+              if (old == marker) {
+                if (*count > kWideWords) break;  // the slab is given up
+                old = atomicCAS(&wt.key[b], marker, cand);
+                if (old == marker) {
+                  wt.at[b] = nidx;
+                  wt.list[atomicAdd(&wt.n, 1)] = (uint16_t)b;
+                  old = cand;
+                }
+              }
+              if (old == cand) break;
+              b = (b + 1) & (kWideBuckets - 1);
+            }
+            slot = b;
+          }
+        }
+        pslot[(r - r0) * cols + c] = (uint16_t)slot;
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    const int used = wt.n;
+    if (used > kWideWords) {  // only a slab of more rows than this, which always fit
+      slab = kWideWords / cols;
+      continue;
+    }
+    // 2. the pairs
+    {
+      const int total = used + (wt.at[WideTab::kMark] != ~0u ? 1 : 0), chunks = (total + 31) / 32;
+      uint16_t *queue = wt.exact[warp];
+      int queued = 0;
+      auto drain = [&](int n) {
+        queued -= n;
+        if (lane < n) {
+          const uint32_t pair = queue[queued + lane];
+          wt.rank[pair >> WideTab::kSlotBits][pair & ((1u << WideTab::kSlotBits) - 1u)] =
+              run_rank((int)run_exact(wt, P.wdesc, s_snap, pair).x);
+        }
+        __syncwarp();
+      };
+#pragma unroll 1
+      for (int t = warp; t < nb * chunks; t += kWarps) {
+        const int c = t / nb, k = t - c * nb, i = 32 * c + lane;
+        bool out = false;
+        uint32_t pair = 0;
+        if (i < total) {
+          const uint32_t s = i < used ? wt.list[i] : WideTab::kMark;
+          pair = (uint32_t)k << WideTab::kSlotBits | s;
+          int e = 0;  // the block's own word: err_diff 0, no refit
+          if (wt.key[s] != wt.own[k]) out = !run_quick(wt, P.wdesc, s_snap, pair, e);
+          wt.rank[k][s] = run_rank(e);
+        }
+        const unsigned om = __ballot_sync(kFull, out);
+        if (out) queue[queued + __popc(om & lt_mask)] = (uint16_t)pair;
+        queued += __popc(om);
+        __syncwarp();
+        if (queued >= 32) drain(32);
+      }
+      if (queued > 0) drain(queued);
+    }
+    __syncthreads();
+    // 3. the selections
+    if (warp < nb) {
+      const uint16_t *rank = wt.rank[warp], *mine = pslot + warp;
+      const int p0 = r0 * w2, npos = (r1 - r0) * w2, drow = 32 / w2, dcol = 32 - drow * w2;
+      const int row0 = lane / w2, col0 = lane - row0 * w2;
+      auto each = [&](auto f) {
+        int at = row0 * cols + col0, col = col0;
+#pragma unroll 4
+        for (int p = lane; p < npos; p += 32) {
+          f((uint32_t)rank[mine[at]], (uint32_t)(p0 + p));
+          at += drow * cols + dcol;
+          col += dcol;
+          if (col >= w2) {
+            col -= w2;
+            at += cols - w2;
+          }
+        }
+      };
+      // rank << 14 | position, in scan order (rows, then columns)
+      uint32_t b = 0xFFFFFFFFu;
+      each([&](uint32_t v, uint32_t p) { b = min(b, (v << 14) | p); });
+      b = __reduce_min_sync(kFull, b);
+      if (b < 1u << 14) {  // an err_diff < 0
+        each([&](uint32_t v, uint32_t p) {
+          if (v <= 1u) first = min(first, p);
+          if (v == 0u) last = max(last, (int)((p / (uint32_t)w2 << 14) | (16383u - p)));
+        });
+      } else if (b < 2u << 14) {  // an err_diff of 0, the first of this slab
+        first = min(first, b & 16383u);
+      }
+      best = min(best, b);
+    }
+    r0 = r1;
+  }
+  if (warp < nb) {
+    int pos = -1;
+    if (best < 2u << 14) {
+      first = __reduce_min_sync(kFull, first);
+      last = __reduce_max_sync(kFull, last);
+      if (P.thr >= 0) pos = last >= 0 && (last >> 14) > (int)(first / (uint32_t)w2) ? 16383 - (last & 16383) : (int)first;
+    } else if (best < kNoRank << 14 && (int)(best >> 14) - 1 <= P.thr) {
+      pos = (int)(best & 16383u);
+    }
+    if (lane == 0) wt.win[warp] = pos;
+  }
+  __syncthreads();
+  if (tid < nb) {
+    const int idx = by * P.bw + bx0 + tid, pos = wt.win[tid];
+    uint64_t word = 0;
+    if (pos >= 0) {
+      const int row = pos / w2, col = pos - row * w2;
+      const uint32_t nidx = (uint32_t)((j0 + row) * P.bw + i0 + tid + col), cand = __ldg(prev_hi + 2 * (size_t)nidx);
+      uint64_t blk = P.stb[idx];
+      if (cand != wt.own[tid]) {
+        wt.key[tid] = cand;  // a slot of the table for the refit
+        wt.at[tid] = nidx;
+        blk = (uint64_t)run_exact(wt, P.wdesc, s_snap, (uint32_t)tid << WideTab::kSlotBits | (uint32_t)tid).y |
+              ((uint64_t)cand << 32);
+      }
+      P.final_blk[idx] = blk;
+      P.motion[idx] = (uint16_t)((col | 0x80) | ((row | 0x80) << 8));
+      word = done_word(blk);
+    }
+    P.done[idx] = word;
   }
 }
 

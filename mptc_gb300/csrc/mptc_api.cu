@@ -234,7 +234,7 @@ enum KernelId {
   K_EMBED_G, K_EMBED_F, K_SCORE, K_EVAL, K_FALLBACK, K_COUNT
 };
 // inter_search: the inter search kernels of an inter frame (inter_run_kernel
-// and inter_overflow_kernel at sa <= 8, inter_dedup_kernel above; the
+// and inter_overflow_kernel at sa <= 8, inter_wide_kernel above; the
 // learned proposal's kernels when a model is attached)
 const char *kKernelNames[K_COUNT] = {"dxt1_encode_kernel",      "inter_search",
                                      "intra_search_kernel",     "intra_sweep_kernel/inter_frame",
@@ -368,26 +368,30 @@ int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int g
   return 1;
 }
 
-// The row pipeline's shared memory (its warps' tables).
-cudaError_t intra_rows_attr() {
-  return cudaFuncSetAttribute(mptc::intra_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(mptc::RowShared));
+// The dynamic shared memory of the row pipeline (its warps' tables) and of the
+// largest window's search.
+cudaError_t search_attrs() {
+  const cudaError_t e = cudaFuncSetAttribute(mptc::intra_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(mptc::RowShared));
+  return e != cudaSuccess ? e
+                          : cudaFuncSetAttribute(mptc::inter_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 mptc::wide_smem(63));
 }
 
-// The exhaustive inter search: one warp per run of kInterRun blocks of a row
-// at sa <= 8 (the runs share the deduplication of their windows; a persistent
+// The exhaustive inter search. sa <= 8: one warp per run of kInterRun blocks
+// of a row (the runs share the deduplication of their windows; a persistent
 // grid of 32 warps per SM takes the runs from the zeroed counter work[7]),
 // then one CTA per block for the blocks of overflowing runs, listed in
-// ovf_list (work[8] of them); one warp per block for larger windows.
+// ovf_list (work[8] of them). Larger windows: one CTA per run.
 // work: the zeroed counter words. Returns the number of kernels launched.
 int launch_inter_search(const mptc::SearchParams &P, int warps, uint32_t *work, uint32_t *ovf_list, int sm_count,
                         cudaStream_t s) {
   const int nblk = P.bw * P.bh;
   if (P.sa > 8) {
-    if (warps == 2)
-      mptc::launch_chain(mptc::inter_dedup_kernel<2>, (nblk + 1) / 2, 2 * 32, s, P);
-    else
-      mptc::launch_chain(mptc::inter_dedup_kernel<4>, (nblk + 3) / 4, 4 * 32, s, P);
+    // shorter runs where a frame has fewer of them than the four CTAs per SM
+    const int slots = 4 * sm_count, run = std::min(mptc::kRun, (nblk + slots - 1) / slots);
+    mptc::launch_chain_smem(mptc::inter_wide_kernel, (P.bw + run - 1) / run * P.bh, mptc::kWideThreads,
+                            mptc::wide_smem(P.sa), s, P, run);
     return 1;
   }
   // runs of kInterRun blocks, in a small frame short enough to give every warp
@@ -720,7 +724,7 @@ mptc_status mptc_ctx_create(const mptc_config *cfg, int32_t width, int32_t heigh
   if (cudaGetDevice(&ctx->device) != cudaSuccess) return bad(MPTC_ECUDA);
   if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess)
     return bad(MPTC_ECUDA);
-  if (ensure_tables(ctx->device) != cudaSuccess || intra_rows_attr() != cudaSuccess) return bad(MPTC_ECUDA);
+  if (ensure_tables(ctx->device) != cudaSuccess || search_attrs() != cudaSuccess) return bad(MPTC_ECUDA);
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mptc::intra_search_kernel<kIntraThreads>,
                                                     kIntraThreads, 0) != cudaSuccess)
@@ -1412,7 +1416,7 @@ mptc_status noalloc_setup(int device, NoallocDevice **out) {
   if (!d.ready) {
     void *p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return MPTC_ECUDA;
-    if (ensure_tables(device) != cudaSuccess || intra_rows_attr() != cudaSuccess) return MPTC_ECUDA;
+    if (ensure_tables(device) != cudaSuccess || search_attrs() != cudaSuccess) return MPTC_ECUDA;
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return MPTC_ECUDA;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mptc::intra_search_kernel<kIntraThreads>,
