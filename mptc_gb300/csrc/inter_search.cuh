@@ -111,11 +111,9 @@ __device__ __forceinline__ uint16_t run_rank(int e) {
   return (uint16_t)(e == kInvalid ? kNoRank : (uint32_t)max(e, -1) + 1u);
 }
 
-// The pixels of a run's nb blocks by one warp, one block row per lane.
-__device__ __forceinline__ void stage_run(PixBlock *px, const SearchParams &P, int bx0, int by, int nb, int lane) {
-  const int k = lane >> 2, r = lane & 3;
-  uint32_t c0 = 0, c1 = 0, c2 = 0;
-  if (k < nb) load_channels(P.rgb, P.width, bx0 + k, 4 * by + r, c0, c1, c2);
+// A block's row of pixels (load_channels) into px by four adjacent lanes, lane r of
+// them row r; every lane of the warp calls it, `store` where its block exists.
+__device__ __forceinline__ void stage_row(PixBlock &px, uint32_t c0, uint32_t c1, uint32_t c2, int r, bool store) {
   uint32_t s0 = __dp4a(c0, 0x01010101u, 0u), s1 = __dp4a(c1, 0x01010101u, 0u), s2 = __dp4a(c2, 0x01010101u, 0u);
   uint32_t sq = __dp4a(c0, c0, __dp4a(c1, c1, __dp4a(c2, c2, 0u)));
 #pragma unroll
@@ -125,12 +123,20 @@ __device__ __forceinline__ void stage_run(PixBlock *px, const SearchParams &P, i
     s2 += __shfl_xor_sync(kFull, s2, o);
     sq += __shfl_xor_sync(kFull, sq, o);
   }
-  if (k < nb) {
-    px[k].pg[0][r] = c0;
-    px[k].pg[1][r] = c1;
-    px[k].pg[2][r] = c2;
-    if (r == 0) *reinterpret_cast<uint4 *>(px[k].sum) = make_uint4(s0, s1, s2, sq);
+  if (store) {
+    px.pg[0][r] = c0;
+    px.pg[1][r] = c1;
+    px.pg[2][r] = c2;
+    if (r == 0) *reinterpret_cast<uint4 *>(px.sum) = make_uint4(s0, s1, s2, sq);
   }
+}
+
+// The pixels of a run's nb blocks by one warp, one block row per lane.
+__device__ __forceinline__ void stage_run(PixBlock *px, const SearchParams &P, int bx0, int by, int nb, int lane) {
+  const int k = lane >> 2, r = lane & 3;
+  uint32_t c0 = 0, c1 = 0, c2 = 0;
+  if (k < nb) load_channels(P.rgb, P.width, bx0 + k, 4 * by + r, c0, c1, c2);
+  stage_row(px[k], c0, c1, c2, r, k < nb);
 }
 
 // SA: the search area when fixed at compile time (its constants fold), 0 to

@@ -489,18 +489,26 @@ __global__ void __launch_bounds__(kScoreThreads, 1) score_topk_tc_kernel(const _
 }
 
 // ---- exact test of the proposals -------------------------------------------------
-// A warp tests the K proposals of 32/K blocks at once (lane = block slot x
-// proposal). Each proposal is evaluated exactly (refit, snap, validity, error;
+// Every proposal is evaluated exactly (refit, snap, validity, error;
 // codec/dxt_image.cpp:258-349) and the reference's selection rule
 // (codec/dxt_image.cpp:715-774: the first err_diff <= 0 in scan order ends its
 // row, a later row's first err_diff < 0 replaces it, otherwise the first
 // minimum) runs over the K proposal positions in closed form. A block whose
 // selection passes the threshold becomes final with the reference's inter
 // motion code; the others are listed for the exhaustive search.
+// A warp takes a group of up to 32 blocks. It evaluates their proposals 32 at a time
+// from the integer sums (refit_quick), the next 32's words loaded meanwhile, and
+// queues the few that need the reference's float steps (refit_exact) for one or
+// two passes at the end, where 32 blocks' near ties fill one better than 4 blocks'
+// would. Results are 16-bit ranks (run_rank) and endpoints per block and
+// proposal; then lane = block selects. Bound by issue. With a table of float
+// products per block, the proposals of 32/K blocks per warp and the selection by
+// shuffles it took 44 us for a 1080p frame's 8 proposals a block, 29 now.
 // The frames of up to kMaxBatch jobs per launch: job j owns the block groups
-// [group_end[j-1], group_end[j]) (a group: the 32/K blocks of one warp pass).
+// [group_end[j-1], group_end[j]) of `group` blocks each.
+constexpr int kEvalWarps = 4, kEvalGroup = 32;
 struct EvalBatch {
-  int n;
+  int n, group;
   int group_end[kMaxBatch];
   SearchParams P[kMaxBatch];
   const uint16_t *topk[kMaxBatch];
@@ -508,104 +516,166 @@ struct EvalBatch {
   uint32_t *fb_list[kMaxBatch];   // room for every block of the frame
 };
 
-template <int K, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) learned_eval_kernel(const __grid_constant__ EvalBatch batch) {
-  constexpr int BPW = 32 / K;
-  __shared__ BlockTab s_tab[WARPS][BPW];
-  __shared__ uint8_t s_snap5[256], s_snap6[256];
-  build_snap_tables(s_snap5, s_snap6);
+template <int K>
+struct EvalTab {
+  PixBlock px[kEvalGroup];
+  int orig[kEvalGroup];
+  uint32_t own[kEvalGroup];
+  uint32_t at[kEvalGroup];       // block row << 16 | column
+  uint16_t pos[kEvalGroup][K];   // window position, kNoProposal where there is none
+  uint16_t rank[kEvalGroup][K];
+  uint32_t eps[kEvalGroup][K];
+  uint16_t exact[kEvalGroup * K];  // block * K + proposal
+};
+
+template <int K>
+__global__ void __launch_bounds__(kEvalWarps * 32, 8) learned_eval_kernel(const __grid_constant__ EvalBatch batch) {
+  __shared__ EvalTab<K> s_tab[kEvalWarps];
+  __shared__ SnapTables s_snap;
+  build_snap_edges(s_snap);
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = lane / K, k = lane % K;
+  depend();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  EvalTab<K> &t = s_tab[warp];
   const int total = batch.group_end[batch.n - 1];
-  for (int gg = blockIdx.x * WARPS + warp; gg < total; gg += gridDim.x * WARPS) {
+  for (int gg = blockIdx.x * kEvalWarps + warp; gg < total; gg += gridDim.x * kEvalWarps) {
     int jb = 0;
     while (gg >= batch.group_end[jb]) ++jb;
     const SearchParams &P = batch.P[jb];
-    const uint16_t *__restrict__ topk = batch.topk[jb];
-    const int nblk = P.bw * P.bh, w2 = 2 * P.sa;
+    const int w2 = 2 * P.sa, bw = P.bw;
     const uint32_t *prev_hi = reinterpret_cast<const uint32_t *>(P.prev) + 1;
-    const int base = (gg - (jb ? batch.group_end[jb - 1] : 0)) * BPW;
-    int sumsq = 0;
-    if constexpr (BPW == 1) {
-      if (base < nblk) {
-        const int by = base / P.bw, bx = base - by * P.bw;
-        sumsq = stage_block(s_tab[warp][0], P.rgb, P.width, bx, by, lane);
-      }
-    } else {
-      // two blocks per staging pass, half a warp each
+    const int base = (gg - (jb ? batch.group_end[jb - 1] : 0)) * batch.group;
+    const int nb = min(batch.group, bw * P.bh - base), idx = base + lane;
+    const uint32_t w2_magic = 0xFFFFFFFFu / (uint32_t)w2 + 1u;  // p / w2 as a multiply-high, exact for p < 2^16
+    const int my_by = idx / bw, my_bx = idx - my_by * bw;
+    t.at[lane] = (uint32_t)my_by << 16 | (uint32_t)my_bx;
+    if (lane < nb) {
+      t.orig[lane] = P.orig_err[idx];
+      t.own[lane] = (uint32_t)(P.stb[idx] >> 32);
+      const uint4 *src = reinterpret_cast<const uint4 *>(batch.topk[jb] + (size_t)idx * kMaxK);
+      if (K == 4) {
+        *reinterpret_cast<uint2 *>(t.pos[lane]) = *reinterpret_cast<const uint2 *>(src);
+      } else {
 #pragma unroll
-      for (int jj = 0; jj < BPW; jj += 2) {
-        const int ia = base + jj, ib = ia + 1;
-        const int ay = ia / P.bw, ax = ia - ay * P.bw, by2 = ib / P.bw, bx2 = ib - by2 * P.bw;
-        const int sq = stage_block_pair(s_tab[warp][jj], s_tab[warp][jj + 1], P.rgb, P.width, ax, ay, ia < nblk,
-                                        bx2, by2, ib < nblk, lane);
-        const int sqa = __shfl_sync(kFull, sq, 0), sqb = __shfl_sync(kFull, sq, 16);
-        if (slot == jj) sumsq = sqa;
-        if (slot == jj + 1) sumsq = sqb;
+        for (int q = 0; q < K / 8; ++q) reinterpret_cast<uint4 *>(t.pos[lane])[q] = src[q];
       }
     }
-    const int idx = base + slot;
-    const bool valid = idx < nblk;
-    const int by = valid ? idx / P.bw : 0, bx = valid ? idx - by * P.bw : 0;
-    const BlockTab &tab = s_tab[warp][slot];
-    int e = kInvalid, pos = -1, refit = 0;
-    uint32_t cand = 0, eps = 0;
-    uint64_t stb = 0;
-    if (valid) {
-      stb = P.stb[idx];
-      const uint16_t p = topk[(size_t)idx * kMaxK + k];
-      const int prow = p / w2, pcol = p - prow * w2;
-      const int gy = by - P.sa + prow, gx = bx - P.sa + pcol;
-      // the scoring kernel lists in-frame window positions only; anything
-      // else (a list left from an aborted launch) is ignored, never read
-      if (p != kNoProposal && p < w2 * w2 && gy >= 0 && gy < P.bh && gx >= 0 && gx < P.bw) {
-        pos = p;
-        const size_t nidx = (size_t)gy * P.bw + gx;
-        cand = __ldg(prev_hi + 2 * nidx);
-        const float4 d = __ldg(P.wdesc + nidx);
-        const WeightSums ws{d.x, d.y, d.z, d.w};
-        const PixelGroups pg = load_groups(tab);
-        e = eval_candidate(tab, pg, s_snap5, s_snap6, cand, ws, (uint32_t)(stb >> 32), P.orig_err[idx], sumsq, eps,
-                           refit);
+    // the blocks' pixels, a block row per lane; all loads first, so that their latencies overlap
+    uint32_t c[kEvalGroup / 8][3] = {};
+#pragma unroll
+    for (int q = 0; q < kEvalGroup / 8; ++q) {
+      const int b = 8 * q + (lane >> 2), by = __shfl_sync(kFull, my_by, b), bx = __shfl_sync(kFull, my_bx, b);
+      if (b < nb) load_channels(P.rgb, P.width, bx, 4 * by + (lane & 3), c[q][0], c[q][1], c[q][2]);
+    }
+#pragma unroll
+    for (int q = 0; q < kEvalGroup / 8; ++q) {
+      const int b = 8 * q + (lane >> 2);
+      stage_row(t.px[b], c[q][0], c[q][1], c[q][2], lane & 3, b < nb);
+    }
+    __syncwarp();
+    // the proposals: pair = block * K + proposal
+    const int pairs = nb * K;
+    struct Word {
+      uint32_t cand;
+      float4 d;
+      bool there;
+    };
+    auto fetch = [&](int pair) {
+      Word w{0u, make_float4(0.f, 0.f, 0.f, 0.f), false};
+      if (pair < pairs) {
+        const int b = pair / K, p = t.pos[b][pair % K], by = (int)(t.at[b] >> 16), bx = (int)(t.at[b] & 0xFFFFu);
+        const int prow = (int)__umulhi((uint32_t)p, w2_magic), gy = by - P.sa + prow, gx = bx - P.sa + p - prow * w2;
+        // the scoring kernel lists in-frame window positions only; anything
+        // else (a list left from an aborted launch) is ignored, never read
+        if (p != kNoProposal && p < w2 * w2 && gy >= 0 && gy < P.bh && gx >= 0 && gx < bw) {
+          const size_t nidx = (size_t)gy * bw + gx;
+          w.cand = __ldg(prev_hi + 2 * nidx);
+          w.d = __ldg(P.wdesc + nidx);
+          w.there = true;
+        }
+      }
+      return w;
+    };
+    int queued = 0;
+    Word next = fetch(lane);
+#pragma unroll 1
+    for (int p0 = 0; p0 < pairs; p0 += 32) {
+      const int pair = p0 + lane, b = min(pair / K, kEvalGroup - 1), k = pair % K;
+      const Word w = next;
+      next = fetch(pair + 32);
+      bool out = false;
+      if (pair < pairs) {
+        uint32_t rank = kNoRank, eps = 0;
+        if (w.there) {
+          if (w.cand == t.own[b]) {
+            rank = 1u;  // err_diff 0, no refit
+          } else {
+            RefitValues r;
+            out = !refit_quick(t.px[b], s_snap, w.cand, WeightSums{w.d.x, w.d.y, w.d.z, w.d.w}, r);
+            rank = run_rank(refit_error(t.px[b], r, w.cand, t.orig[b], eps));
+          }
+        }
+        t.rank[b][k] = (uint16_t)rank;
+        t.eps[b][k] = eps;
+      }
+      const unsigned om = __ballot_sync(kFull, out);
+      if (out) t.exact[queued + __popc(om & lt_mask)] = (uint16_t)pair;
+      queued += __popc(om);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int q0 = 0; q0 < queued; q0 += 32) {
+      if (q0 + lane < queued) {
+        const int pair = t.exact[q0 + lane], b = pair / K, k = pair % K;
+        const Word w = fetch(pair);
+        RefitValues r;
+        uint32_t eps;
+        refit_exact(t.px[b], s_snap, w.cand, WeightSums{w.d.x, w.d.y, w.d.z, w.d.w}, r);
+        t.rank[b][k] = run_rank(refit_error(t.px[b], r, w.cand, t.orig[b], eps));
+        t.eps[b][k] = eps;
       }
     }
-    const int row = pos >= 0 ? pos / w2 : 0;
-    // P0: first position with err_diff <= 0
-    int k1 = (e != kInvalid && e <= 0) ? pos : 0xFFFF;
+    __syncwarp();
+    // lane = block: the selection
+    bool open = false;
+    if (lane < nb) {
+      int first = 0xFFFF, last = -1, sel = -1;  // last: row << 16 | 0xFFFF - position
+      uint32_t best = 0xFFFFFFFFu;              // rank << 16 | position
 #pragma unroll
-    for (int o = K / 2; o > 0; o >>= 1) k1 = min(k1, __shfl_xor_sync(kFull, k1, o));
-    const int r0 = k1 < 0xFFFF ? k1 / w2 : 0x7FFF;
-    // the last later row with an err_diff < 0, and its first such position
-    int k2 = (e != kInvalid && e < 0 && row > r0) ? (row << 16) | (0xFFFF - pos) : 0;
+      for (int k = 0; k < K; ++k) {
+        const uint32_t v = t.rank[lane][k];
+        const int p = t.pos[lane][k];
+        if (v <= 1u) first = min(first, p);
+        if (v == 0u) last = max(last, (int)(__umulhi((uint32_t)p, w2_magic) << 16) | (0xFFFF - p));
+        if (v != kNoRank) best = min(best, v << 16 | (uint32_t)p);
+      }
+      if (first != 0xFFFF) {
+        if (P.thr >= 0) sel = (last >> 16) > first / w2 ? 0xFFFF - (last & 0xFFFF) : first;
+      } else if (best != 0xFFFFFFFFu && (int)(best >> 16) - 1 <= P.thr) {
+        sel = (int)(best & 0xFFFFu);
+      }
+      uint64_t word = 0;
+      if (sel >= 0) {
+        uint32_t eps = 0;
 #pragma unroll
-    for (int o = K / 2; o > 0; o >>= 1) k2 = max(k2, __shfl_xor_sync(kFull, k2, o));
-    // otherwise the first minimum
-    int k3 = e != kInvalid ? ((e + 65536) << 12) | pos : 0x7FFFFFFF;
-#pragma unroll
-    for (int o = K / 2; o > 0; o >>= 1) k3 = min(k3, __shfl_xor_sync(kFull, k3, o));
-    int sel = -1, m = kInvalid;
-    if (k2 > 0) {
-      sel = 0xFFFF - (k2 & 0xFFFF);
-      m = 0;
-    } else if (k1 < 0xFFFF) {
-      sel = k1;
-      m = 0;
-    } else if (k3 != 0x7FFFFFFF) {
-      sel = k3 & 0xFFF;
-      m = (k3 >> 12) - 65536;
+        for (int k = 0; k < K; ++k)
+          if (t.pos[lane][k] == sel) eps = t.eps[lane][k];
+        const int row = sel / w2, col = sel - row * w2;
+        const uint32_t cand = __ldg(prev_hi + 2 * ((size_t)(my_by - P.sa + row) * bw + my_bx - P.sa + col));
+        const uint64_t blk = cand == t.own[lane] ? P.stb[idx] : (uint64_t)eps | ((uint64_t)cand << 32);
+        P.final_blk[idx] = blk;
+        P.motion[idx] = (uint16_t)((col | 0x80) | ((row | 0x80) << 8));
+        word = done_word(blk);
+      }
+      P.done[idx] = word;
+      open = word == 0;
     }
-    const bool accept = sel >= 0 && m <= P.thr;
-    if (valid && accept && pos == sel) {
-      const uint64_t blk = refit ? ((uint64_t)eps | ((uint64_t)cand << 32)) : stb;
-      const int col = sel - row * w2;
-      P.final_blk[idx] = blk;
-      P.motion[idx] = (uint16_t)((col | 0x80) | ((row | 0x80) << 8));
-      P.done[idx] = done_word(blk);
-    }
-    if (valid && !accept && k == 0) {
-      P.done[idx] = 0;
-      batch.fb_list[jb][atomicAdd(batch.fb_count[jb], 1u)] = (uint32_t)idx;
-    }
+    const unsigned om = __ballot_sync(kFull, open);
+    uint32_t at = 0;
+    if (lane == 0 && om) at = atomicAdd(batch.fb_count[jb], (uint32_t)__popc(om));
+    at = __shfl_sync(kFull, at, 0);
+    if (open) batch.fb_list[jb][at + __popc(om & lt_mask)] = (uint32_t)idx;
     __syncwarp();
   }
 }
@@ -626,6 +696,8 @@ struct ListBatch {
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) inter_list_kernel(const __grid_constant__ ListBatch batch) {
   static_assert(THREADS >= 256, "one thread per position of a 16x16 window");
+  depend();
+  release_next();
   int total = 0;
   for (int j = 0; j < batch.n; ++j) total += (int)__ldcg(batch.count[j]);
   if ((int)blockIdx.x >= total) return;  // the whole CTA, before its barriers

@@ -475,9 +475,8 @@ void launch_score(const mptc::ScoreBatch &sb, int sm_count, cudaStream_t s) {
 
 template <int K>
 void launch_eval(const mptc::EvalBatch &eb, int sm_count, cudaStream_t s) {
-  constexpr int WARPS = 4;
-  const int grid = std::min((eb.group_end[eb.n - 1] + WARPS - 1) / WARPS, sm_count * 16);
-  mptc::learned_eval_kernel<K, WARPS><<<grid, WARPS * 32, 0, s>>>(eb);
+  const int grid = std::min((eb.group_end[eb.n - 1] + mptc::kEvalWarps - 1) / mptc::kEvalWarps, sm_count * 16);
+  mptc::launch_chain(mptc::learned_eval_kernel<K>, grid, mptc::kEvalWarps * 32, s, eb);
 }
 
 // The g half of the learned search for up to kMaxBatch previous frames
@@ -572,8 +571,12 @@ int launch_learned(const LearnedJob *jobs, int n, uint32_t *counters, cudaStream
   mptc::ListBatch lb{};
   lb.n = n;
   const bool r8 = c0->score_rows == 8;  // 128- or 64-entry palette slices
-  const int bpw = 32 / c0->topk_k;
-  int tiles = 0, groups = 0;
+  // groups of 32 blocks a warp, of 16 or 8 where that leaves the SMs fewer than 24
+  // warps each
+  int tiles = 0, groups = 0, blocks = 0;
+  for (int j = 0; j < n; ++j) blocks += jobs[j].ctx->nblk;
+  eb.group = mptc::kEvalGroup;
+  while (eb.group > 8 && blocks < eb.group * 24 * c0->sm_count) eb.group /= 2;
   for (int j = 0; j < n; ++j) {
     mptc_ctx *c = jobs[j].ctx;
     tiles += ((c->bw + mptc::kScoreTileW - 1) / mptc::kScoreTileW) *
@@ -582,7 +585,7 @@ int launch_learned(const LearnedJob *jobs, int n, uint32_t *counters, cudaStream
     sb.a[j] = mptc::ScoreArgs{c->bw, c->bh, c->cfg.search_area, reinterpret_cast<const uint32_t *>(jobs[j].P.prev) + 1,
                               2, c->gemb, c->dict_rows, c->topk, c->work + 1};
     sb.tmF[j] = c->tm_f;
-    groups += (c->nblk + bpw - 1) / bpw;
+    groups += (c->nblk + eb.group - 1) / eb.group;
     eb.group_end[j] = groups;
     eb.P[j] = jobs[j].P;
     eb.topk[j] = c->topk;
@@ -611,7 +614,7 @@ int launch_learned(const LearnedJob *jobs, int n, uint32_t *counters, cudaStream
   }
   {
     KernelTimer t(c0, K_FALLBACK, s);
-    mptc::inter_list_kernel<256><<<sms * 4, 256, 0, s>>>(lb);  // CTAs past the lists' end return at once
+    mptc::launch_chain(mptc::inter_list_kernel<256>, sms * 4, 256, s, lb);  // CTAs past the lists' end return at once
   }
   return 6;
 }
