@@ -71,6 +71,10 @@ __device__ __forceinline__ uint64_t ld_shared_relaxed(const uint64_t *p) {
 // word it is, so that its refit weight sums are read (P.wdesc[src]) instead of
 // summed again.
 //
+// Several frames at once are bound by the SMs that their CTAs hold: with two CTAs per
+// SM (96 registers, a table of 768 buckets instead of 1024) the first frames of 8
+// streams up to 2560x1440 and their 15 learned inter frames take 25.3 ms, with one 27.9.
+//
 // Bound by latency: the critical path of an intra frame is bw + sa * bh steps
 // from a block to its right neighbour or to the row below, here about 0.2 us
 // and 1 us, with one warp's chains of dependent instructions (about 5 cycles
@@ -87,7 +91,7 @@ constexpr int kRowCols = kRowGroup + 15 + kRowBack;  // union columns at sa = 8
 constexpr int kRowOld = 12;               // rows y-4 .. y-15
 // At most 12 * 31 words of step A, 55 without a position, 3 * 31 of rows y-3 ..
 // y-1 and 15 left neighbours: the table never fills.
-constexpr int kRowBuckets = 1024;
+constexpr int kRowBuckets = 768;
 constexpr int kRowAll = 128;  // up to so many words of step A are evaluated on every block
 constexpr uint16_t kNoBucket = 0xFFFFu;
 constexpr uint32_t kNoMatch = 0x100u;  // above every position
@@ -138,7 +142,10 @@ struct RowShared {
 
 static_assert(sizeof(RowDict) % 16 == 0 && offsetof(RowWork, ent) % 16 == 0 && offsetof(RowMail, later) % 16 == 0, "vector stores reset the tables");
 
-__device__ __forceinline__ uint32_t row_hash(uint32_t w) { return (w * 2654435761u) >> 22; }
+__device__ __forceinline__ uint32_t row_hash(uint32_t w) {
+  return __umulhi(w * 2654435761u, (uint32_t)kRowBuckets);
+}
+__device__ __forceinline__ uint32_t row_after(uint32_t b) { return b + 1u < (uint32_t)kRowBuckets ? b + 1u : 0u; }
 // The tag of group g's words (never 0 on the row's first lap).
 __device__ __forceinline__ uint64_t row_tag(int g) { return (uint64_t)((g + 1) & 31) << 59; }
 template <class T>
@@ -186,7 +193,7 @@ __device__ __forceinline__ uint32_t row_enter(RowDict &D, uint64_t w, bool &is_n
     const unsigned long long old = atomicCAS(&D.key[b], 0ull, (unsigned long long)w);
     is_new = old == 0ull;
     if (is_new || (uint32_t)old == (uint32_t)w) break;
-    b = (b + 1) & (kRowBuckets - 1);
+    b = row_after(b);
   }
   return b;
 }
@@ -202,7 +209,7 @@ __device__ __forceinline__ bool row_find(const RowDict &D, const RowWork &W, uin
       e = (int)(uint32_t)(v >> 32);
       return (uint32_t)v == word;
     }
-    b = (b + 1) & (kRowBuckets - 1);
+    b = row_after(b);
   }
   return false;
 }
@@ -486,7 +493,7 @@ __device__ __forceinline__ void row_worker(RowShared &S, const SearchParams &P, 
     if (p != kNoMatch && word != own) {
       uint32_t b = row_hash(word);
       for (int probe = 0; probe < kRowBuckets && (uint32_t)ld_volatile(&D.key[b]) != word; ++probe)
-        b = (b + 1) & (kRowBuckets - 1);
+        b = row_after(b);
       blk = (uint64_t)ld_volatile(&W.eps[b]) | ((uint64_t)word << 32);
     }
     P.final_blk[idx] = blk;
@@ -548,7 +555,11 @@ __device__ __noinline__ RowAnswer row_decide(RowShared &S, const SearchParams &P
   return r;
 }
 
-__global__ void __launch_bounds__(kRowThreads, 1) intra_rows_kernel(SearchParams P) {
+// PER_SM: CTAs that an SM holds at once. A frame by itself is fastest with one (two
+// of its CTAs on an SM slow the chain: 1.81 ms against 1.51 at 1080p); frames
+// beside others' take half the registers and share the SMs.
+template <int PER_SM>
+__global__ void __launch_bounds__(kRowThreads, PER_SM) intra_rows_kernel(SearchParams P) {
   extern __shared__ __align__(16) uint8_t row_smem[];
   RowShared &S = *reinterpret_cast<RowShared *>(row_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -612,7 +623,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) intra_rows_kernel(SearchParams
             mb = ld_shared_v4(&M->later);
             unsigned long long v = ld_volatile(reinterpret_cast<const unsigned long long *>(&W->ent[hb]));
             const unsigned long long v2 = ld_volatile(
-                reinterpret_cast<const unsigned long long *>(&W->ent[(hb + 1) & (kRowBuckets - 1)]));
+                reinterpret_cast<const unsigned long long *>(&W->ent[row_after(hb)]));
             if ((uint32_t)v != lo) v = v2;
             const bool wait = ((tag ^ ma.y) >> 27) != 0u;
             m = __reduce_min_sync(kFull, on ? ((uint32_t)max((int)(v >> 32), 0) << 5) | (uint32_t)lane : 0xFFFFFFFFu);

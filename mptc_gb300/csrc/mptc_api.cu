@@ -342,10 +342,17 @@ int launch_begin(const mptc::SearchParams &P, float4 *wdesc, int ntiles, bool ch
   return 1;
 }
 
+// More shared memory than half an SM's: one CTA of the row pipeline per SM.
+constexpr int kRowsAlone = 120 * 1024;
+static_assert(2 * (sizeof(mptc::RowShared) + 1024) <= 228 * 1024 && sizeof(mptc::RowShared) <= kRowsAlone,
+              "two CTAs of the row pipeline share an SM");
+
 // The intra search of a whole intra frame, behind launch_begin: the row pipeline
-// on `ctas` SMs at sa <= 8, the block dataflow on `grid` CTAs for larger windows.
+// with `ctas` CTAs at sa <= 8 (alone: one per SM; otherwise beside other frames, two
+// per SM), the block dataflow on `grid` CTAs for larger windows.
 // Returns the number of kernels launched.
-int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int grid, int ctas, cudaStream_t s) {
+int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int grid, int ctas, bool alone,
+                       cudaStream_t s) {
   const int nblk = P.bw * P.bh;
   if (P.sa > 8) {
     mptc::intra_search_kernel<kIntraThreads><<<grid, kIntraThreads, 0, s>>>(P, order, nullptr, nblk);
@@ -354,7 +361,7 @@ int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int g
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(mptc::kRowCluster * std::max(1, std::min(P.bh, ctas / mptc::kRowCluster)));
   cfg.blockDim = dim3(mptc::kRowThreads);
-  cfg.dynamicSmemBytes = sizeof(mptc::RowShared);
+  cfg.dynamicSmemBytes = alone ? kRowsAlone : sizeof(mptc::RowShared);
   cfg.stream = s;
   cudaLaunchAttribute at[2]{};
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -364,18 +371,21 @@ int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int g
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, mptc::intra_rows_kernel, P);
+  cudaLaunchKernelEx(&cfg, alone ? mptc::intra_rows_kernel<1> : mptc::intra_rows_kernel<2>, P);
   return 1;
 }
 
 // The dynamic shared memory of the row pipeline (its warps' tables) and of the
 // largest window's search.
 cudaError_t search_attrs() {
-  const cudaError_t e = cudaFuncSetAttribute(mptc::intra_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(mptc::RowShared));
-  return e != cudaSuccess ? e
-                          : cudaFuncSetAttribute(mptc::inter_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 mptc::wide_smem(63));
+  cudaError_t e = cudaFuncSetAttribute(mptc::intra_rows_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kRowsAlone);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(mptc::intra_rows_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(mptc::RowShared));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(mptc::inter_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mptc::wide_smem(63));
+  return e;
 }
 
 // The exhaustive inter search. sa <= 8: one warp per run of kInterRun blocks
@@ -671,7 +681,7 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
     else
       ctx->launches += launch_intra_frame(P, ctx->order, ig,
                                           ctx->intra_cap > 0 ? std::min(ctx->intra_cap, ctx->sm_count) : ctx->sm_count,
-                                          s);
+                                          ctx->intra_cap <= 0, s);
   }
   MPTC_CUDA(cudaGetLastError());
   const uint16_t *m16 = P.motion;
@@ -1503,7 +1513,7 @@ extern "C" mptc_status mptc_encode_frame_noalloc(const mptc_config *cfg, int32_t
                  work + 5, sweep, sweep + 3 * (size_t)n, sw ? sw + 1 : 0, work + 1);
     launch_intra_sweeps(P, pend, work + 5, sweep, n, d->intra_grid, sw, sweep_part, kSweepPartCapNoalloc, s);
   } else {
-    launch_intra_frame(P, order, d->intra_grid, d->sm_count, s);
+    launch_intra_frame(P, order, d->intra_grid, d->sm_count, true, s);
   }
   const uint16_t *m16 = reinterpret_cast<const uint16_t *>(motion_dev);
   mptc::launch_chain(mptc::unique_scan_kernel, ntiles, 256, s, m16, stb, n, ntiles, tile_state + ntiles, work + 11,
@@ -1649,6 +1659,7 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
     mptc_status st = lane_init(c);
     if (st != MPTC_OK) return st;
     c->lane_b->timing = c->timing;
+    c->lane_b->intra_cap = c->sm_count;  // the lanes share the SMs with each other first (half each: 26.1 ms, not 25.3)
     c->lane_b->model = nullptr;  // intra frames: no inter search
     while ((int)b->lane_ev[i].size() < n_frames) {
       cudaEvent_t e;
