@@ -358,6 +358,31 @@ __device__ __forceinline__ void refit_exact(const PixBlock &t, const SnapTables 
   }
 }
 
+// One channel of it: the pixels' bytes, the channel's snap table; entries of ep1's and
+// ep2's value.
+__device__ __forceinline__ void refit_exact_channel(const uint32_t (&pg)[4], const uint32_t *snap, uint32_t cand,
+                                                    const WeightSums &ws, uint32_t &snap1, uint32_t &snap2) {
+  const float third = __fdiv_rn(1.0f, 3.0f), third2 = __fadd_rn(third, third);
+  float ax = 0.f, bx = 0.f;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const uint32_t w = pg[g], idx = cand >> (8 * g);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t k = (idx >> (2 * i)) & 3u;
+      const float lo = (k & 2u) ? third2 : 1.0f, hi = (k & 2u) ? third : 0.0f;
+      const float fa = (k & 1u) ? hi : lo, fb = (k & 1u) ? lo : hi;
+      const float px = __uint2float_rn((w >> (8 * i)) & 0xFFu);
+      ax = __fadd_rn(ax, __fmul_rn(px, fa));
+      bx = __fadd_rn(bx, __fmul_rn(px, fb));
+    }
+  }
+  const float p1 = __fmul_rn(ws.f, __fsub_rn(__fmul_rn(ax, ws.bsq), __fmul_rn(bx, ws.ab)));
+  const float p2 = __fmul_rn(ws.f, __fsub_rn(__fmul_rn(bx, ws.asq), __fmul_rn(ax, ws.ab)));
+  snap1 = snap[quantize_endpoint(__fadd_rn(p1, 0.5f))];
+  snap2 = snap[quantize_endpoint(__fadd_rn(p2, 0.5f))];
+}
+
 // err_diff of the refitted candidate (kInvalid where its endpoints would swap)
 // and its packed endpoints.
 __device__ __forceinline__ int refit_error(const PixBlock &t, const RefitValues &r, uint32_t cand, int orig_err,
@@ -387,6 +412,40 @@ __device__ __forceinline__ int refit_error(const PixBlock &t, const RefitValues 
   }
   const int sse = (int)t.sumsq - 2 * (int)cross + (int)norm;
   return q1 > q2 ? (int)((uint32_t)sse / 48u) - orig_err : kInvalid;
+}
+
+// refit_exact and refit_error of up to kByChannels candidates by a warp, a lane per
+// channel: few candidates need the float steps, and a pass with a lane per
+// candidate costs as much for one as for 32 (560 instructions against 330). get(q):
+// candidate q of n; returns candidate `lane`'s err_diff and endpoints. All lanes call.
+constexpr int kByChannels = 10;
+struct ExactCase {
+  const PixBlock *px;
+  uint32_t cand;
+  float4 d;  // its weight sums
+  int orig;
+};
+template <class Get>
+__device__ __forceinline__ uint2 refit_by_channels(const SnapTables &st, int n, int lane, Get get) {
+  const int q = lane / 3, c = lane - 3 * q;
+  uint32_t v1 = 0, v2 = 0;
+  if (q < n) {
+    const ExactCase x = get(q);
+    refit_exact_channel(x.px->pg[c], c == 1 ? st.six : st.five, x.cand, WeightSums{x.d.x, x.d.y, x.d.z, x.d.w}, v1, v2);
+  }
+  RefitValues r;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    r.snap[k] = __shfl_sync(kFull, v1, 3 * lane + k);
+    r.snap[3 + k] = __shfl_sync(kFull, v2, 3 * lane + k);
+  }
+  uint32_t eps = 0;
+  int e = kInvalid;
+  if (lane < n) {
+    const ExactCase x = get(lane);
+    e = refit_error(*x.px, r, x.cand, x.orig, eps);
+  }
+  return make_uint2((uint32_t)e, eps);
 }
 
 }  // namespace mptc

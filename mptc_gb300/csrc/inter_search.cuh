@@ -107,6 +107,12 @@ __device__ __forceinline__ uint2 run_exact(const Tab &rt, const float4 *wdesc, c
   const int e = refit_error(rt.px[k], r, rt.key[s], rt.orig[k], eps);
   return make_uint2((uint32_t)e, eps);
 }
+// Pair q of a run for refit_by_channels.
+template <class Tab>
+__device__ __forceinline__ ExactCase run_case(const Tab &rt, const float4 *wdesc, uint32_t pair) {
+  const int k = (int)(pair >> Tab::kSlotBits), s = (int)(pair & ((1u << Tab::kSlotBits) - 1u));
+  return ExactCase{&rt.px[k], rt.key[s], __ldg(wdesc + rt.at[s]), rt.orig[k]};
+}
 __device__ __forceinline__ uint16_t run_rank(int e) {
   return (uint16_t)(e == kInvalid ? kNoRank : (uint32_t)max(e, -1) + 1u);
 }
@@ -313,7 +319,17 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
           nexact += __popc(om);
           __syncwarp();
         }
-        if (nexact >= 32 || (last && nquick == 0 && nexact > 0)) {
+        if (last && nquick == 0 && nexact > 0 && nexact <= kByChannels) {
+          const int n = nexact;
+          nexact = 0;
+          const uint2 x =
+              refit_by_channels(s_snap, n, lane, [&](int q) { return run_case(rt, P.wdesc, rt.exact[q]); });
+          if (lane < n) {
+            const uint32_t pair = rt.exact[lane];
+            rt.rank[pair >> 8][pair & 255u] = run_rank((int)x.x);
+          }
+          __syncwarp();
+        } else if (nexact >= 32 || (last && nquick == 0 && nexact > 0)) {
           const int n = min(nexact, 32);
           nexact -= n;
           if (lane < n) {
@@ -365,15 +381,18 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
       if (lane == k && pos >= 0)
         win = ((uint32_t)pos + 1u) << 8 | pslot[pos / w2 * Tab::kStride + pos % w2];
     }
+    // the selected words' endpoints (a block's own word needs none: computed, unused)
+    if (lane < nb) rt.exact[lane] = (uint16_t)((uint32_t)lane << 8 | (win & 255u));
+    __syncwarp();
+    const uint2 refit =
+        refit_by_channels(s_snap, nb, lane, [&](int q) { return run_case(rt, P.wdesc, rt.exact[q]); });
     if (lane < nb) {
       const int idx = by * P.bw + bx0 + lane;
       uint64_t word = 0;
       if (win != 0u) {
         const uint32_t s = win & 255u, pos = (win >> 8) - 1u;
         uint64_t blk = P.stb[idx];
-        if (rt.key[s] != rt.own[lane]) {
-          blk = (uint64_t)run_exact(rt, P.wdesc, s_snap, (uint32_t)lane << 8 | s).y | ((uint64_t)rt.key[s] << 32);
-        }
+        if (rt.key[s] != rt.own[lane]) blk = (uint64_t)refit.y | ((uint64_t)rt.key[s] << 32);
         const uint32_t row = pos / (uint32_t)w2, col = pos - row * (uint32_t)w2;
         P.final_blk[idx] = blk;
         P.motion[idx] = (uint16_t)((col | 0x80) | ((row | 0x80) << 8));
@@ -547,7 +566,15 @@ __global__ void __launch_bounds__(kWideThreads, 4) inter_wide_kernel(SearchParam
         __syncwarp();
         if (queued >= 32) drain(32);
       }
-      if (queued > 0) drain(queued);
+      if (queued > kByChannels) {
+        drain(queued);
+      } else if (queued > 0) {
+        const uint2 x = refit_by_channels(s_snap, queued, lane, [&](int q) { return run_case(wt, P.wdesc, queue[q]); });
+        if (lane < queued) {
+          const uint32_t pair = queue[lane];
+          wt.rank[pair >> WideTab::kSlotBits][pair & ((1u << WideTab::kSlotBits) - 1u)] = run_rank((int)x.x);
+        }
+      }
     }
     __syncthreads();
     // 3. the selections
@@ -596,19 +623,29 @@ __global__ void __launch_bounds__(kWideThreads, 4) inter_wide_kernel(SearchParam
     if (lane == 0) wt.win[warp] = pos;
   }
   __syncthreads();
-  if (tid < nb) {
-    const int idx = by * P.bw + bx0 + tid, pos = wt.win[tid];
+  if (warp != 0) return;
+  // the selected words' endpoints (a block's own word needs none: computed, unused);
+  // each word in a slot of the table
+  const int pos = lane < nb ? wt.win[lane] : -1, row = max(pos, 0) / w2, col = max(pos, 0) - row * w2;
+  uint32_t cand = marker;
+  if (pos >= 0) {
+    const uint32_t nidx = (uint32_t)((j0 + row) * P.bw + i0 + lane + col);
+    cand = __ldg(prev_hi + 2 * (size_t)nidx);
+    wt.at[lane] = nidx;
+  } else if (lane < nb) {
+    wt.at[lane] = 0;
+  }
+  if (lane < nb) wt.key[lane] = cand;
+  __syncwarp();
+  const uint2 refit = refit_by_channels(s_snap, nb, lane, [&](int q) {
+    return run_case(wt, P.wdesc, (uint32_t)q << WideTab::kSlotBits | (uint32_t)q);
+  });
+  if (lane < nb) {
+    const int idx = by * P.bw + bx0 + lane;
     uint64_t word = 0;
     if (pos >= 0) {
-      const int row = pos / w2, col = pos - row * w2;
-      const uint32_t nidx = (uint32_t)((j0 + row) * P.bw + i0 + tid + col), cand = __ldg(prev_hi + 2 * (size_t)nidx);
       uint64_t blk = P.stb[idx];
-      if (cand != wt.own[tid]) {
-        wt.key[tid] = cand;  // a slot of the table for the refit
-        wt.at[tid] = nidx;
-        blk = (uint64_t)run_exact(wt, P.wdesc, s_snap, (uint32_t)tid << WideTab::kSlotBits | (uint32_t)tid).y |
-              ((uint64_t)cand << 32);
-      }
+      if (cand != wt.own[lane]) blk = (uint64_t)refit.y | ((uint64_t)cand << 32);
       P.final_blk[idx] = blk;
       P.motion[idx] = (uint16_t)((col | 0x80) | ((row | 0x80) << 8));
       word = done_word(blk);

@@ -624,6 +624,19 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 8) learned_eval_kernel(const 
       queued += __popc(om);
     }
     __syncwarp();
+    if (queued > 0 && queued <= kByChannels) {
+      const uint2 x = refit_by_channels(s_snap, queued, lane, [&](int q) {
+        const int pair = t.exact[q];
+        const Word w = fetch(pair);
+        return ExactCase{&t.px[pair / K], w.cand, w.d, t.orig[pair / K]};
+      });
+      if (lane < queued) {
+        const int pair = t.exact[lane];
+        t.rank[pair / K][pair % K] = run_rank((int)x.x);
+        t.eps[pair / K][pair % K] = x.y;
+      }
+      queued = 0;
+    }
 #pragma unroll 1
     for (int q0 = 0; q0 < queued; q0 += 32) {
       if (q0 + lane < queued) {
