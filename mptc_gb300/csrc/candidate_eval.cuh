@@ -252,10 +252,22 @@ __device__ __forceinline__ int eval_candidate(const BlockTab &t, const PixelGrou
 constexpr float kRefitRel = 1.46e-6f;  // > 23.1u (1.05 x)
 constexpr float kRefitAbs = 1.0e-4f;   // > 260 * 5u + 2^-16
 
-struct __align__(16) PixBlock {
-  uint32_t pg[3][4];  // channel c bytes of pixels 4g .. 4g+3
-  uint32_t sum[3];    // sum of channel c
-  uint32_t sumsq;     // sum of squares over all channels
+// The pixels of N blocks: [0 .. 2][block] the channel's bytes of pixels 4g .. 4g+3 in
+// word g, [3][block] the channels' sums, then the sum of squares over all. A
+// vector of adjacent blocks is contiguous, so lanes that work on different blocks
+// read it without bank conflicts (a block by itself, 64 bytes, put every other
+// block into the same banks: 11 million conflicts a 1080p frame).
+template <int N>
+struct __align__(16) PixBlocks {
+  uint32_t w[4][N][4];
+};
+// Block k of them.
+template <int N>
+struct PixBlock {
+  const PixBlocks<N> &t;
+  int k;
+  __device__ __forceinline__ uint4 vec(int c) const { return *reinterpret_cast<const uint4 *>(t.w[c][k]); }
+  __device__ __forceinline__ uint32_t word(int c, int g) const { return t.w[c][k][g]; }
 };
 
 // The snap tables with, per value, whether the snapped value differs from that
@@ -294,22 +306,24 @@ struct RefitValues {
 };
 
 // From the exact sums; false where the float steps may give another value.
-__device__ __forceinline__ bool refit_quick(const PixBlock &t, const SnapTables &st, uint32_t cand,
+template <int N>
+__device__ __forceinline__ bool refit_quick(const PixBlock<N> t, const SnapTables &st, uint32_t cand,
                                             const WeightSums &ws, RefitValues &r) {
   const float third = __fdiv_rn(1.0f, 3.0f);
   uint32_t ord[4];
 #pragma unroll
   for (int g = 0; g < 4; ++g) ord[g] = __byte_perm(0x02010300u, 0u, spread_nibbles((cand >> (8 * g)) & 0xFFu));
-  const float tmax = __uint2float_rn(max(t.sum[0], max(t.sum[1], t.sum[2])));
+  const uint4 sums = t.vec(3);
+  const uint32_t sum[3] = {sums.x, sums.y, sums.z};
+  const float tmax = __uint2float_rn(max(sum[0], max(sum[1], sum[2])));
   const float margin =
       __fmaf_rn(__fmul_rn(__fmul_rn(kRefitRel, tmax), fabsf(ws.f)), fmaxf(ws.asq, ws.bsq), kRefitAbs);
   uint32_t edge = 0;  // bit 31: a value within the margin of an integer where its snapped value changes
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    uint32_t S = 0;
-#pragma unroll
-    for (int g = 0; g < 4; ++g) S = __dp4a(t.pg[c][g], ord[g], S);
-    const float b = __fmul_rn(__uint2float_rn(S), third), a = __fmul_rn(__uint2float_rn(3u * t.sum[c] - S), third);
+    const uint4 pg = t.vec(c);
+    const uint32_t S = __dp4a(pg.w, ord[3], __dp4a(pg.z, ord[2], __dp4a(pg.y, ord[1], __dp4a(pg.x, ord[0], 0u))));
+    const float b = __fmul_rn(__uint2float_rn(S), third), a = __fmul_rn(__uint2float_rn(3u * sum[c] - S), third);
     const float v1 = __fmaf_rn(ws.f, __fsub_rn(__fmul_rn(a, ws.bsq), __fmul_rn(b, ws.ab)), 0.5f);
     const float v2 = __fmaf_rn(ws.f, __fsub_rn(__fmul_rn(b, ws.asq), __fmul_rn(a, ws.ab)), 0.5f);
 #pragma unroll
@@ -327,13 +341,14 @@ __device__ __forceinline__ bool refit_quick(const PixBlock &t, const SnapTables 
 }
 
 // By the reference's own steps (codec/dxt_image.cpp:298-331).
-__device__ __forceinline__ void refit_exact(const PixBlock &t, const SnapTables &st, uint32_t cand,
+template <int N>
+__device__ __forceinline__ void refit_exact(const PixBlock<N> t, const SnapTables &st, uint32_t cand,
                                             const WeightSums &ws, RefitValues &r) {
   const float third = __fdiv_rn(1.0f, 3.0f), third2 = __fadd_rn(third, third);
   float ax[3] = {0.f, 0.f, 0.f}, bx[3] = {0.f, 0.f, 0.f};
 #pragma unroll 1
   for (int g = 0; g < 4; ++g) {
-    const uint32_t w[3] = {t.pg[0][g], t.pg[1][g], t.pg[2][g]}, idx = cand >> (8 * g);
+    const uint32_t w[3] = {t.word(0, g), t.word(1, g), t.word(2, g)}, idx = cand >> (8 * g);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint32_t k = (idx >> (2 * i)) & 3u;
@@ -360,13 +375,13 @@ __device__ __forceinline__ void refit_exact(const PixBlock &t, const SnapTables 
 
 // One channel of it: the pixels' bytes, the channel's snap table; entries of ep1's and
 // ep2's value.
-__device__ __forceinline__ void refit_exact_channel(const uint32_t (&pg)[4], const uint32_t *snap, uint32_t cand,
+__device__ __forceinline__ void refit_exact_channel(uint4 pg, const uint32_t *snap, uint32_t cand,
                                                     const WeightSums &ws, uint32_t &snap1, uint32_t &snap2) {
   const float third = __fdiv_rn(1.0f, 3.0f), third2 = __fadd_rn(third, third);
   float ax = 0.f, bx = 0.f;
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
-    const uint32_t w = pg[g], idx = cand >> (8 * g);
+    const uint32_t w = g == 0 ? pg.x : g == 1 ? pg.y : g == 2 ? pg.z : pg.w, idx = cand >> (8 * g);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint32_t k = (idx >> (2 * i)) & 3u;
@@ -385,7 +400,8 @@ __device__ __forceinline__ void refit_exact_channel(const uint32_t (&pg)[4], con
 
 // err_diff of the refitted candidate (kInvalid where its endpoints would swap)
 // and its packed endpoints.
-__device__ __forceinline__ int refit_error(const PixBlock &t, const RefitValues &r, uint32_t cand, int orig_err,
+template <int N>
+__device__ __forceinline__ int refit_error(const PixBlock<N> t, const RefitValues &r, uint32_t cand, int orig_err,
                                            uint32_t &eps) {
   const uint32_t q1 = ((r.snap[0] << 8) & 0xF800u) | ((r.snap[1] << 3) & 0x07E0u) | ((r.snap[2] >> 3) & 0x1Fu);
   const uint32_t q2 = ((r.snap[3] << 8) & 0xF800u) | ((r.snap[4] << 3) & 0x07E0u) | ((r.snap[5] >> 3) & 0x1Fu);
@@ -400,17 +416,18 @@ __device__ __forceinline__ int refit_error(const PixBlock &t, const RefitValues 
     pal[c] = ends | ((x2 * (683u << 5)) & 0x00FF0000u) | ((x3 * (683u << 13)) & 0xFF000000u);
   }
   uint32_t cross = 0, norm = 0;
+  const uint4 pg[3] = {t.vec(0), t.vec(1), t.vec(2)};
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     const uint32_t sel = spread_nibbles((cand >> (8 * g)) & 0xFFu);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const uint32_t v = __byte_perm(pal[c], 0u, sel);
-      cross = __dp4a(t.pg[c][g], v, cross);
+      cross = __dp4a(g == 0 ? pg[c].x : g == 1 ? pg[c].y : g == 2 ? pg[c].z : pg[c].w, v, cross);
       norm = __dp4a(v, v, norm);
     }
   }
-  const int sse = (int)t.sumsq - 2 * (int)cross + (int)norm;
+  const int sse = (int)t.word(3, 3) - 2 * (int)cross + (int)norm;
   return q1 > q2 ? (int)((uint32_t)sse / 48u) - orig_err : kInvalid;
 }
 
@@ -419,8 +436,9 @@ __device__ __forceinline__ int refit_error(const PixBlock &t, const RefitValues 
 // candidate costs as much for one as for 32 (560 instructions against 330). get(q):
 // candidate q of n; returns candidate `lane`'s err_diff and endpoints. All lanes call.
 constexpr int kByChannels = 10;
+template <int N>
 struct ExactCase {
-  const PixBlock *px;
+  PixBlock<N> px;
   uint32_t cand;
   float4 d;  // its weight sums
   int orig;
@@ -430,8 +448,8 @@ __device__ __forceinline__ uint2 refit_by_channels(const SnapTables &st, int n, 
   const int q = lane / 3, c = lane - 3 * q;
   uint32_t v1 = 0, v2 = 0;
   if (q < n) {
-    const ExactCase x = get(q);
-    refit_exact_channel(x.px->pg[c], c == 1 ? st.six : st.five, x.cand, WeightSums{x.d.x, x.d.y, x.d.z, x.d.w}, v1, v2);
+    const auto x = get(q);
+    refit_exact_channel(x.px.vec(c), c == 1 ? st.six : st.five, x.cand, WeightSums{x.d.x, x.d.y, x.d.z, x.d.w}, v1, v2);
   }
   RefitValues r;
 #pragma unroll
@@ -442,8 +460,8 @@ __device__ __forceinline__ uint2 refit_by_channels(const SnapTables &st, int n, 
   uint32_t eps = 0;
   int e = kInvalid;
   if (lane < n) {
-    const ExactCase x = get(lane);
-    e = refit_error(*x.px, r, x.cand, x.orig, eps);
+    const auto x = get(lane);
+    e = refit_error(x.px, r, x.cand, x.orig, eps);
   }
   return make_uint2((uint32_t)e, eps);
 }

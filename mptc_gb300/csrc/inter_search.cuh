@@ -60,7 +60,7 @@ struct RunTab {
   // row that crosses the limit
   static constexpr int kSlots = 1 + kRunWords + kCols;
   static constexpr int kSentinel = kSlots;  // slot of out-of-frame positions
-  PixBlock px[kRun];
+  PixBlocks<kRun> px;
   int orig[kRun];
   uint32_t own[kRun];
   union {
@@ -91,8 +91,8 @@ __device__ __forceinline__ bool run_quick(const Tab &rt, const float4 *wdesc, co
   const WeightSums ws{d.x, d.y, d.z, d.w};
   RefitValues r;
   uint32_t eps;
-  const bool ok = refit_quick(rt.px[k], st, rt.key[s], ws, r);
-  e = refit_error(rt.px[k], r, rt.key[s], rt.orig[k], eps);
+  const bool ok = refit_quick(PixBlock<kRun>{rt.px, k}, st, rt.key[s], ws, r);
+  e = refit_error(PixBlock<kRun>{rt.px, k}, r, rt.key[s], rt.orig[k], eps);
   return ok;
 }
 // Evaluates a pair by the reference's own steps: its err_diff and endpoints.
@@ -103,23 +103,25 @@ __device__ __forceinline__ uint2 run_exact(const Tab &rt, const float4 *wdesc, c
   const WeightSums ws{d.x, d.y, d.z, d.w};
   RefitValues r;
   uint32_t eps;
-  refit_exact(rt.px[k], st, rt.key[s], ws, r);
-  const int e = refit_error(rt.px[k], r, rt.key[s], rt.orig[k], eps);
+  refit_exact(PixBlock<kRun>{rt.px, k}, st, rt.key[s], ws, r);
+  const int e = refit_error(PixBlock<kRun>{rt.px, k}, r, rt.key[s], rt.orig[k], eps);
   return make_uint2((uint32_t)e, eps);
 }
 // Pair q of a run for refit_by_channels.
 template <class Tab>
-__device__ __forceinline__ ExactCase run_case(const Tab &rt, const float4 *wdesc, uint32_t pair) {
+__device__ __forceinline__ ExactCase<kRun> run_case(const Tab &rt, const float4 *wdesc, uint32_t pair) {
   const int k = (int)(pair >> Tab::kSlotBits), s = (int)(pair & ((1u << Tab::kSlotBits) - 1u));
-  return ExactCase{&rt.px[k], rt.key[s], __ldg(wdesc + rt.at[s]), rt.orig[k]};
+  return ExactCase<kRun>{PixBlock<kRun>{rt.px, k}, rt.key[s], __ldg(wdesc + rt.at[s]), rt.orig[k]};
 }
 __device__ __forceinline__ uint16_t run_rank(int e) {
   return (uint16_t)(e == kInvalid ? kNoRank : (uint32_t)max(e, -1) + 1u);
 }
 
-// A block's row of pixels (load_channels) into px by four adjacent lanes, lane r of
+// Block k's row of pixels (load_channels) into px by four adjacent lanes, lane r of
 // them row r; every lane of the warp calls it, `store` where its block exists.
-__device__ __forceinline__ void stage_row(PixBlock &px, uint32_t c0, uint32_t c1, uint32_t c2, int r, bool store) {
+template <int N>
+__device__ __forceinline__ void stage_row(PixBlocks<N> &px, int k, uint32_t c0, uint32_t c1, uint32_t c2, int r,
+                                          bool store) {
   uint32_t s0 = __dp4a(c0, 0x01010101u, 0u), s1 = __dp4a(c1, 0x01010101u, 0u), s2 = __dp4a(c2, 0x01010101u, 0u);
   uint32_t sq = __dp4a(c0, c0, __dp4a(c1, c1, __dp4a(c2, c2, 0u)));
 #pragma unroll
@@ -130,19 +132,19 @@ __device__ __forceinline__ void stage_row(PixBlock &px, uint32_t c0, uint32_t c1
     sq += __shfl_xor_sync(kFull, sq, o);
   }
   if (store) {
-    px.pg[0][r] = c0;
-    px.pg[1][r] = c1;
-    px.pg[2][r] = c2;
-    if (r == 0) *reinterpret_cast<uint4 *>(px.sum) = make_uint4(s0, s1, s2, sq);
+    px.w[0][k][r] = c0;
+    px.w[1][k][r] = c1;
+    px.w[2][k][r] = c2;
+    if (r == 0) *reinterpret_cast<uint4 *>(px.w[3][k]) = make_uint4(s0, s1, s2, sq);
   }
 }
 
 // The pixels of a run's nb blocks by one warp, one block row per lane.
-__device__ __forceinline__ void stage_run(PixBlock *px, const SearchParams &P, int bx0, int by, int nb, int lane) {
+__device__ __forceinline__ void stage_run(PixBlocks<kRun> &px, const SearchParams &P, int bx0, int by, int nb, int lane) {
   const int k = lane >> 2, r = lane & 3;
   uint32_t c0 = 0, c1 = 0, c2 = 0;
   if (k < nb) load_channels(P.rgb, P.width, bx0 + k, 4 * by + r, c0, c1, c2);
-  stage_row(px[k], c0, c1, c2, r, k < nb);
+  stage_row(px, k, c0, c1, c2, r, k < nb);
 }
 
 // SA: the search area when fixed at compile time (its constants fold), 0 to
@@ -431,7 +433,7 @@ struct WideTab {
   static constexpr int kSlotBits = 11;
   static constexpr int kMark = kWideBuckets;      // slot of the empty buckets' word, the first block's own
   static constexpr int kNone = kWideBuckets + 1;  // slot of out-of-frame positions
-  PixBlock px[kRun];
+  PixBlocks<kRun> px;
   int orig[kRun];
   uint32_t own[kRun];
   uint32_t key[kWideBuckets + 1];

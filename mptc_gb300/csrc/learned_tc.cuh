@@ -518,7 +518,7 @@ struct EvalBatch {
 
 template <int K>
 struct EvalTab {
-  PixBlock px[kEvalGroup];
+  PixBlocks<kEvalGroup> px;
   int orig[kEvalGroup];
   uint32_t own[kEvalGroup];
   uint32_t at[kEvalGroup];       // block row << 16 | column
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 8) learned_eval_kernel(const 
 #pragma unroll
     for (int q = 0; q < kEvalGroup / 8; ++q) {
       const int b = 8 * q + (lane >> 2);
-      stage_row(t.px[b], c[q][0], c[q][1], c[q][2], lane & 3, b < nb);
+      stage_row(t.px, b, c[q][0], c[q][1], c[q][2], lane & 3, b < nb);
     }
     __syncwarp();
     // the proposals: pair = block * K + proposal
@@ -612,8 +612,8 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 8) learned_eval_kernel(const 
             rank = 1u;  // err_diff 0, no refit
           } else {
             RefitValues r;
-            out = !refit_quick(t.px[b], s_snap, w.cand, WeightSums{w.d.x, w.d.y, w.d.z, w.d.w}, r);
-            rank = run_rank(refit_error(t.px[b], r, w.cand, t.orig[b], eps));
+            out = !refit_quick(PixBlock<kEvalGroup>{t.px, b}, s_snap, w.cand, WeightSums{w.d.x, w.d.y, w.d.z, w.d.w}, r);
+            rank = run_rank(refit_error(PixBlock<kEvalGroup>{t.px, b}, r, w.cand, t.orig[b], eps));
           }
         }
         t.rank[b][k] = (uint16_t)rank;
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 8) learned_eval_kernel(const 
       const uint2 x = refit_by_channels(s_snap, queued, lane, [&](int q) {
         const int pair = t.exact[q];
         const Word w = fetch(pair);
-        return ExactCase{&t.px[pair / K], w.cand, w.d, t.orig[pair / K]};
+        return ExactCase<kEvalGroup>{PixBlock<kEvalGroup>{t.px, pair / K}, w.cand, w.d, t.orig[pair / K]};
       });
       if (lane < queued) {
         const int pair = t.exact[lane];
@@ -644,8 +644,8 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 8) learned_eval_kernel(const 
         const Word w = fetch(pair);
         RefitValues r;
         uint32_t eps;
-        refit_exact(t.px[b], s_snap, w.cand, WeightSums{w.d.x, w.d.y, w.d.z, w.d.w}, r);
-        t.rank[b][k] = run_rank(refit_error(t.px[b], r, w.cand, t.orig[b], eps));
+        refit_exact(PixBlock<kEvalGroup>{t.px, b}, s_snap, w.cand, WeightSums{w.d.x, w.d.y, w.d.z, w.d.w}, r);
+        t.rank[b][k] = run_rank(refit_error(PixBlock<kEvalGroup>{t.px, b}, r, w.cand, t.orig[b], eps));
         t.eps[b][k] = eps;
       }
     }
