@@ -247,7 +247,7 @@ __device__ __forceinline__ int eval_candidate(const BlockTab &t, const PixelGrou
 // (the same in both) add 4u of ax * bsq + bx * ab, which is at most
 // T * max(asq, bsq): |difference| <= 23.1u * |f| * T * max(asq, bsq) + 5u * |p| plus
 // the two roundings of p + 0.5 (each <= 2^-17). |p| <= 260 covers every value that
-// the clamp to [0, 255] leaves. Where that is not below a half (a degenerate
+// the clamp to [0, 255] leaves. Where that is not below a quarter (a degenerate
 // word, all indices equal: f huge, infinite or NaN), refit_exact decides.
 constexpr float kRefitRel = 1.46e-6f;  // > 23.1u (1.05 x)
 constexpr float kRefitAbs = 1.0e-4f;   // > 260 * 5u + 2^-16
@@ -271,19 +271,16 @@ struct PixBlock {
 };
 
 // The snap tables with, per value, whether the snapped value differs from that
-// of the value before (bit 31) and after (bit 30); the snapped value in the low
-// byte.
-constexpr uint32_t kSnapLow = 0x80000000u, kSnapHigh = 0x40000000u;
+// of the value before (bit 31); the snapped value in the low byte.
+constexpr uint32_t kSnapLow = 0x80000000u;
 struct SnapTables {
   uint32_t five[256], six[256];
 };
 __device__ __forceinline__ void build_snap_edges(SnapTables &t) {
   for (int i = threadIdx.x; i < 512; i += blockDim.x) {
     const uint32_t x = (uint32_t)i & 255u, keep = i < 256 ? 0xF8u : 0xFCu, step = i < 256 ? 4u : 2u, sh = i < 256 ? 5u : 6u;
-    uint32_t v = snap_value(x, keep, step, sh);
-    const uint32_t lo = x > 0u ? snap_value(x - 1u, keep, step, sh) : v, hi = x < 255u ? snap_value(x + 1u, keep, step, sh) : v;
-    const uint32_t e = v | (lo != v ? kSnapLow : 0u) | (hi != v ? kSnapHigh : 0u);
-    (i < 256 ? t.five : t.six)[x] = e;
+    const uint32_t v = snap_value(x, keep, step, sh), lo = x > 0u ? snap_value(x - 1u, keep, step, sh) : v;
+    (i < 256 ? t.five : t.six)[x] = v | (lo != v ? kSnapLow : 0u);
   }
 }
 
@@ -318,7 +315,13 @@ __device__ __forceinline__ bool refit_quick(const PixBlock<N> t, const SnapTable
   const float tmax = __uint2float_rn(max(sum[0], max(sum[1], sum[2])));
   const float margin =
       __fmaf_rn(__fmul_rn(__fmul_rn(kRefitRel, tmax), fabsf(ws.f)), fmaxf(ws.asq, ws.bsq), kRefitAbs);
-  uint32_t edge = 0;  // bit 31: a value within the margin of an integer where its snapped value changes
+  // Values as w + 2048, whose last 12 bits are w's fraction (rounded by half a unit,
+  // which `near`, the margin in units, covers: one unit for its own rounding down,
+  // one for this). With k = floor(w + margin), a fraction of w + margin of at
+  // least twice the margin puts the reference's value at k as well; below that it is k
+  // or k - 1, which is no matter where both snap to the same value.
+  const uint32_t near = (uint32_t)__float2int_rz(__fmul_rn(margin, 4096.0f)) + 2u, span = 2u * near;
+  uint32_t edge = 0;  // bit 31: a value that may be k or k - 1 where they snap differently
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const uint4 pg = t.vec(c);
@@ -329,15 +332,13 @@ __device__ __forceinline__ bool refit_quick(const PixBlock<N> t, const SnapTable
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const float w = fminf(fmaxf(h ? v2 : v1, 0.5f), 255.5f);
-      const float m = __fadd_rd(w, 8388608.0f);  // floor(w) in the low bits
-      const float frac = __fsub_rn(w, __fsub_rn(m, 8388608.0f));
-      const uint32_t e = (c == 1 ? st.six : st.five)[__float_as_uint(m) & 0xFFu];
-      edge |= (__float_as_uint(__fsub_rn(frac, margin)) & e) |
-              (__float_as_uint(__fsub_rn(__fsub_rn(1.0f, margin), frac)) & (e << 1));
+      const uint32_t x = __float_as_uint(__fadd_rn(w, 2048.0f)) + near;
+      const uint32_t e = (c == 1 ? st.six : st.five)[(x >> 12) & 0xFFu];
+      edge |= ((x & 0xFFFu) - span) & e;
       r.snap[3 * h + c] = e;
     }
   }
-  return (int)edge >= 0 && margin < 0.5f;  // false for a NaN or infinite margin
+  return (int)edge >= 0 && margin < 0.25f;  // false for a NaN or infinite margin
 }
 
 // By the reference's own steps (codec/dxt_image.cpp:298-331).
