@@ -352,7 +352,7 @@ static_assert(2 * (sizeof(mptc::RowShared) + 1024) <= 228 * 1024 && sizeof(mptc:
 // per SM), the block dataflow on `grid` CTAs for larger windows.
 // Returns the number of kernels launched.
 int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int grid, int ctas, bool alone,
-                       cudaStream_t s) {
+                       bool chained, cudaStream_t s) {
   const int nblk = P.bw * P.bh;
   if (P.sa > 8) {
     mptc::intra_search_kernel<kIntraThreads><<<grid, kIntraThreads, 0, s>>>(P, order, nullptr, nblk);
@@ -370,7 +370,7 @@ int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int g
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = chained ? 2 : 1;
   cudaLaunchKernelEx(&cfg, alone ? mptc::intra_rows_kernel<1> : mptc::intra_rows_kernel<2>, P);
   return 1;
 }
@@ -624,7 +624,10 @@ int launch_learned(const LearnedJob *jobs, int n, uint32_t *counters, cudaStream
   }
   {
     KernelTimer t(c0, K_FALLBACK, s);
-    mptc::launch_chain(mptc::inter_list_kernel<256>, sms * 4, 256, s, lb);  // CTAs past the lists' end return at once
+    // CTAs past the lists' end return at once; twice those that the SMs hold, so that
+    // a long list's blocks go to whichever SM is free (8 streams' lists: 25.0 ms a run
+    // with 12 per SM, 25.3 with 4)
+    mptc::launch_chain(mptc::inter_list_kernel<256>, sms * 12, 256, s, lb);
   }
   return 6;
 }
@@ -652,9 +655,10 @@ mptc_status reencode_begin(mptc_ctx *ctx, const mptc::SearchParams &P, bool chai
 
 // Last part, after the inter search: an inter frame's pending compaction and
 // intra pass (sweeps + exact fallback), an intra frame's dataflow; the unique
-// palette.
+// palette. chained: the kernel of this frame before it is the one before it in the
+// stream, with no event wait between.
 mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t *unique_dev, uint32_t *n_unique_dev,
-                            cudaStream_t s) {
+                            bool chained, cudaStream_t s) {
   const uint64_t *prev_final_dev = P.prev;
   if (prev_final_dev) {
     // pending = blocks the inter pass left open, in wavefront order, with
@@ -662,7 +666,7 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
     const int sw = sweep_count(ctx->cfg.intra_sweeps);
     uint32_t *changed = ctx->sweep + 3 * (size_t)ctx->nblk;
     const int flags = sw ? sw + 1 : 0;
-    if (ctx->model)  // in a batch behind an event wait
+    if (!chained)  // behind an event wait
       mptc::pending_scan_kernel<<<ctx->ntiles, 256, 0, s>>>(ctx->order, ctx->done, P.stb, ctx->nblk, ctx->ntiles,
                                                            ctx->tile_state, ctx->work + 10, ctx->pending,
                                                            ctx->work + 5, ctx->sweep, changed, flags, ctx->work + 1);
@@ -681,7 +685,7 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
     else
       ctx->launches += launch_intra_frame(P, ctx->order, ig,
                                           ctx->intra_cap > 0 ? std::min(ctx->intra_cap, ctx->sm_count) : ctx->sm_count,
-                                          ctx->intra_cap <= 0, s);
+                                          ctx->intra_cap <= 0, chained, s);
   }
   MPTC_CUDA(cudaGetLastError());
   const uint16_t *m16 = P.motion;
@@ -856,7 +860,7 @@ static mptc_status reencode_run(mptc_ctx *ctx, const uint8_t *rgb_dev, const uin
     }
     MPTC_CUDA(cudaGetLastError());
   }
-  return reencode_finish(ctx, P, unique_dev, n_unique_dev, s);
+  return reencode_finish(ctx, P, unique_dev, n_unique_dev, true, s);
 }
 
 mptc_status mptc_reencode(mptc_ctx *ctx, const uint8_t *rgb_dev, const uint64_t *stb_dev, const int32_t *orig_err_dev,
@@ -1513,7 +1517,7 @@ extern "C" mptc_status mptc_encode_frame_noalloc(const mptc_config *cfg, int32_t
                  work + 5, sweep, sweep + 3 * (size_t)n, sw ? sw + 1 : 0, work + 1);
     launch_intra_sweeps(P, pend, work + 5, sweep, n, d->intra_grid, sw, sweep_part, kSweepPartCapNoalloc, s);
   } else {
-    launch_intra_frame(P, order, d->intra_grid, d->sm_count, true, s);
+    launch_intra_frame(P, order, d->intra_grid, d->sm_count, true, true, s);
   }
   const uint16_t *m16 = reinterpret_cast<const uint16_t *>(motion_dev);
   mptc::launch_chain(mptc::unique_scan_kernel, ntiles, 256, s, m16, stb, n, ntiles, tile_state + ntiles, work + 11,
@@ -1600,7 +1604,7 @@ mptc_status batch_launch(mptc_batch *b, const int32_t *is_intra, int parity, cud
   for (int i = 0; i < b->n; ++i) {
     cudaStream_t si = b->streams[i];
     if (!jobs.empty() && cudaStreamWaitEvent(si, b->learned_ev, 0) != cudaSuccess) return MPTC_ECUDA;
-    mptc_status st = reencode_finish(b->ctx[i], P[i], b->unique[i], b->n_unique + i, si);
+    mptc_status st = reencode_finish(b->ctx[i], P[i], b->unique[i], b->n_unique + i, jobs.empty(), si);
     if (st != MPTC_OK) return st;
     if (cudaEventRecord(b->done_ev[i], si) != cudaSuccess) return MPTC_ECUDA;
     if (cudaStreamWaitEvent(s, b->done_ev[i], 0) != cudaSuccess) return MPTC_ECUDA;
@@ -1751,7 +1755,7 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
       cudaStream_t si = b->streams[i];
       const size_t n = (size_t)c->nblk;
       if (c->model && !jobs.empty() && cudaStreamWaitEvent(si, b->learned_ev, 0) != cudaSuccess) return MPTC_ECUDA;
-      mptc_status st = reencode_finish(c, P[i], uni[i] + k * n, n_uni[i] + k, si);
+      mptc_status st = reencode_finish(c, P[i], uni[i] + k * n, n_uni[i] + k, jobs.empty(), si);
       if (st != MPTC_OK) return st;
       mptc::launch_chain(status_or_kernel, 1, 32, si, c->work, b->run_status);
       if (cudaEventRecord(c->stb_free[slot[i]], si) != cudaSuccess) return MPTC_ECUDA;
