@@ -314,7 +314,8 @@ int launch_intra_sweeps(const mptc::SearchParams &P, const uint32_t *pending, co
   uint32_t *est[3] = {sweep, sweep + n, sweep + 2 * (size_t)n}, *changed = sweep + 3 * (size_t)n;
   for (int k = 0; k < sweeps; ++k)
     mptc::launch_chain(mptc::intra_sweep_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, est[k % 3],
-                 est[(k + 2) % 3], est[(k + 1) % 3], changed + k, changed + k + 1, part, part_cap, k == 0);
+                 est[(k + 2) % 3], est[(k + 1) % 3], changed + k, changed + k + 1, part, part_cap, k == 0,
+                 k == 1 ? n_pending : k == 2 ? changed + 1 : nullptr);
   mptc::launch_chain(mptc::intra_search_kernel<kIntraThreads>, grid, kIntraThreads, s, P, pending, n_pending, -1,
                changed + sweeps);
   return sweeps + 1;
