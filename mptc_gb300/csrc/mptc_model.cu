@@ -167,13 +167,13 @@ cudaError_t ensure_gemm_attrs() {
 // columns where N has no more, or where 128 would leave an SM without a tile.
 template <bool TA, bool TB>
 void gemm(const bf16 *A, int lda, const bf16 *B, int ldb, const mptc::GemmEpi &e, int M, int N, int K, int splits,
-          uint32_t *status, cudaStream_t s) {
+          uint32_t *status, cudaStream_t s, bool chained = true) {
   const int rows = (M + mptc::kTcBM - 1) / mptc::kTcBM, steps = mptc::tc_steps(K, splits);
   if (N <= 64 || rows * ((N + 127) / 128) * splits < 152)
-    mptc::launch_chain_smem(mptc::gemm_tc_kernel<TA, TB, 64>, dim3((N + 63) / 64, rows, splits), 128,
+    mptc::launch_if_chained(chained, mptc::gemm_tc_kernel<TA, TB, 64>, dim3((N + 63) / 64, rows, splits), 128,
                             mptc::tc_smem<64>(steps), s, A, lda, B, ldb, e, M, N, K, status);
   else
-    mptc::launch_chain_smem(mptc::gemm_tc_kernel<TA, TB, 128>, dim3((N + 127) / 128, rows, splits), 128,
+    mptc::launch_if_chained(chained, mptc::gemm_tc_kernel<TA, TB, 128>, dim3((N + 127) / 128, rows, splits), 128,
                             mptc::tc_smem<128>(steps), s, A, lda, B, ldb, e, M, N, K, status);
 }
 
@@ -211,9 +211,9 @@ void gemm_dw(const bf16 *x, const bf16 *dy, float *dW, int M, int K, int N, Sums
 // into dxb (bf16), and the partial column sums of that dx, whose total is db[K]
 // (the bias gradient of the layer below).
 void gemm_dx(const bf16 *dy, const bf16 *W, const bf16 *h, bf16 *dxb, float *db, int M, int K, int N, Sums &sums,
-             uint32_t *status, cudaStream_t s) {
+             uint32_t *status, cudaStream_t s, bool chained = true) {
   float *part = sums.add((M + mptc::kTcBM - 1) / mptc::kTcBM, K, db);
-  gemm<false, true>(dy, N, W, N, {nullptr, dxb, K, nullptr, 0, h, part}, M, K, N, 1, status, s);
+  gemm<false, true>(dy, N, W, N, {nullptr, dxb, K, nullptr, 0, h, part}, M, K, N, 1, status, s, chained);
 }
 
 // Forward through both MLPs for a training batch; then, if `grads`, the loss
@@ -262,7 +262,7 @@ mptc_status forward_backward(mptc_model *m, const uint8_t *rgb, int width, int b
   ok = cudaEventRecord(m->ev[0], s) == cudaSuccess && cudaStreamWaitEvent(t, m->ev[0], 0) == cudaSuccess && ok;
   if (!ok) return MPTC_ECUDA;
   // block MLP
-  gemm_dx(m->dfb, W[2], m->h2b, m->dh2b, Gb[1], B, kH2, kEmb, sums, status, t);
+  gemm_dx(m->dfb, W[2], m->h2b, m->dh2b, Gb[1], B, kH2, kEmb, sums, status, t, false);  // behind an event wait
   gemm_dx(m->dh2b, W[1], m->h1b, m->dh1b, Gb[0], B, kH1, kH2, sums, status, t);
   gemm_dw(m->h2b, m->dfb, G[2], B, kH2, kEmb, sums, status, t);
   gemm_dw(m->h1b, m->dh2b, G[1], B, kH1, kH2, sums, status, t);
