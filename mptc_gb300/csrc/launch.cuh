@@ -41,10 +41,11 @@ void launch_chain(void (*kernel)(Par...), dim3 grid, int threads, cudaStream_t s
 template <typename... Par, typename... Arg>
 void launch_after(void (*kernel)(Par...), dim3 grid, int threads, cudaStream_t s, Arg... arg) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone)
-    launch_chain(kernel, grid, threads, s, arg...);
-  else
-    kernel<<<grid, threads, 0, s>>>(Par(arg)...);
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();  // the launch itself reports what is wrong
+    st = cudaStreamCaptureStatusActive;
+  }
+  launch_if_chained(st == cudaStreamCaptureStatusNone, kernel, grid, threads, 0, s, arg...);
 }
 
 }  // namespace mptc

@@ -76,6 +76,8 @@ class Decoder:
                 with torch.cuda.stream(s):  # staging copies ordered with the decode kernels
                     dst.copy_(torch.from_numpy(src) if isinstance(src, np.ndarray) else src)
                 src = dst
+            elif stream is not None and dst.numel():
+                src.record_stream(s)  # it may be freed on its own stream before s has read it
             ptrs.append(src.data_ptr() if dst.numel() else 0)
         prev = self._frames[self._cur].data_ptr() if self._cur >= 0 else None
         self._cur = (self._cur + 1) % 2

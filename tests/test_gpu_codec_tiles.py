@@ -203,3 +203,33 @@ def test_decoder_input_forms(torch_cuda, form):
             dec.decode_frame(t[0].cuda().view(-1, 2), t[1].cuda(), t[2].cuda())
     finally:
         dec.close()
+
+
+def test_decoder_on_another_stream(torch_cuda):
+    """Inputs read in place on a stream that is not their own, freed and overwritten
+    right after the call."""
+    from mptc_gb300.decoder import Decoder
+    torch = torch_cuda
+    rng = np.random.default_rng(8)
+    n, sa = 64 * 64, 8
+    coeff = rng.integers(0, 256, 6 * n, dtype=np.uint8)
+    motion = codes(rng, "mixed", 64, 64, sa, True).reshape(-1)
+    palette = rng.integers(0, 1 << 32, int((motion.reshape(-1, 2) == 255).all(1).sum()), dtype=np.uint32)
+    host = [torch.from_numpy(a.copy()) for a in (motion, coeff, palette.view(np.int32))]
+    dec, s = Decoder(256, 256, sa), torch.cuda.Stream()
+    try:
+        want = dec.decode_frame(*[x.cuda() for x in host]).cpu()
+        for _ in range(4):
+            args = [x.cuda() for x in host]
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                torch.cuda._sleep(2000000)  # the decode starts after the inputs are gone
+            got = dec.decode_frame(*args, stream=s)
+            shapes = [a.shape for a in args]
+            del args
+            junk = [torch.full(sh, 77, dtype=x.dtype, device="cuda") for sh, x in zip(shapes, host)]
+            s.synchronize()
+            assert torch.equal(got.cpu(), want)
+            del junk
+    finally:
+        dec.close()
