@@ -521,7 +521,7 @@ struct EvalTab {
   PixBlocks<kEvalGroup> px;
   int orig[kEvalGroup];
   uint32_t own[kEvalGroup];
-  uint32_t at[kEvalGroup];       // block row << 16 | column
+  int bx[kEvalGroup];            // block column
   uint16_t pos[kEvalGroup][K];   // window position, kNoProposal where there is none
   uint16_t rank[kEvalGroup][K];
   uint32_t eps[kEvalGroup][K];
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 8) learned_eval_kernel(const 
     const int nb = min(batch.group, bw * P.bh - base), idx = base + lane;
     const uint32_t w2_magic = 0xFFFFFFFFu / (uint32_t)w2 + 1u;  // p / w2 as a multiply-high, exact for p < 2^16
     const int my_by = idx / bw, my_bx = idx - my_by * bw;
-    t.at[lane] = (uint32_t)my_by << 16 | (uint32_t)my_bx;
+    t.bx[lane] = my_bx;
     if (lane < nb) {
       t.orig[lane] = P.orig_err[idx];
       t.own[lane] = (uint32_t)(P.stb[idx] >> 32);
@@ -584,12 +584,15 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 8) learned_eval_kernel(const 
     auto fetch = [&](int pair) {
       Word w{0u, make_float4(0.f, 0.f, 0.f, 0.f), false};
       if (pair < pairs) {
-        const int b = pair / K, p = t.pos[b][pair % K], by = (int)(t.at[b] >> 16), bx = (int)(t.at[b] & 0xFFFFu);
-        const int prow = (int)__umulhi((uint32_t)p, w2_magic), gy = by - P.sa + prow, gx = bx - P.sa + p - prow * w2;
+        // a position's row by its first block, row0 + (prow - sa) bw: a frame may have
+        // more block rows or columns than 16 bits hold
+        const int b = pair / K, p = t.pos[b][pair % K], bx = t.bx[b], row0 = base + b - bx;
+        const int prow = (int)__umulhi((uint32_t)p, w2_magic), gx = bx - P.sa + p - prow * w2;
         // the scoring kernel lists in-frame window positions only; anything
         // else (a list left from an aborted launch) is ignored, never read
-        if (p != kNoProposal && p < w2 * w2 && gy >= 0 && gy < P.bh && gx >= 0 && gx < bw) {
-          const size_t nidx = (size_t)gy * bw + gx;
+        const int row = p < w2 * w2 ? row0 + (prow - P.sa) * bw : -1;
+        if (p != kNoProposal && row >= 0 && row < bw * P.bh && gx >= 0 && gx < bw) {
+          const size_t nidx = (size_t)row + gx;
           w.cand = __ldg(prev_hi + 2 * nidx);
           w.d = __ldg(P.wdesc + nidx);
           w.there = true;
