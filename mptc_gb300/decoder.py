@@ -69,10 +69,12 @@ class Decoder:
             unique = unique.view(np.int32) if isinstance(unique, np.ndarray) else unique.view(torch.int32)
         ptrs = []
         for dst, src in ((self._motion, motion), (self._coeff, coeff), (self._unique[:n_unique], unique)):
-            # a plain CUDA tensor of the kernels' layout is read where it is; three copies
-            # a frame took longer than the decode (61 us a 2048x1280 frame, 38 now)
+            # a plain CUDA tensor of the kernels' layout and length is read where it is (a
+            # palette of another element size has another length as 32-bit words, which
+            # copy_ refuses); three copies a frame took longer than the decode (61 us a
+            # 2048x1280 frame, 38 now)
             if dst.numel() and not (type(src) is torch.Tensor and src.dtype == dst.dtype and src.device == dst.device
-                                    and src.dim() == 1 and src.is_contiguous()):
+                                    and src.shape == dst.shape and src.is_contiguous()):
                 with torch.cuda.stream(s):  # staging copies ordered with the decode kernels
                     dst.copy_(torch.from_numpy(src) if isinstance(src, np.ndarray) else src)
                 src = dst
