@@ -381,7 +381,8 @@ mptc_status mptc_decode_frame(mptc_decoder *dec, const uint8_t *coeff_dev, const
 /* Synchronises `stream` and returns MPTC_EINVAL if any frame decoded since the
  * last check held an invalid motion code (a copy from outside the previous
  * frame or from a block not yet decoded) or a unique count that differs from
- * n_unique; *flags (may be NULL) gets bit 0 / bit 1 for those. Clears them. */
+ * n_unique; *flags (may be NULL) gets bit 0 / bit 1 for those. MPTC_ESTATE if a
+ * frame ran at the same time as another of the same decoder. Clears them. */
 mptc_status mptc_decoder_check(mptc_decoder *dec, void *stream, uint32_t *flags);
 const char *mptc_decoder_last_error(const mptc_decoder *dec);
 

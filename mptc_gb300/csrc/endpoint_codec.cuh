@@ -346,6 +346,10 @@ __global__ void __launch_bounds__(kCodecThreads) decode_parts_kernel(
   if (tid == 0) s_tile = (int)atomicAdd(claim, 1u);
   __syncthreads();
   const int tile = s_tile, i0 = tile * kScanTile + 4 * tid;
+  if ((unsigned)tile >= (unsigned)ntiles) {  // two frames of a decoder at the same time, for instance
+    if (tid == 0) atomicOr(status, kDevBadScan);
+    return;
+  }
   unsigned uq = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -390,7 +394,8 @@ __global__ void __launch_bounds__(kCodecThreads) decode_parts_kernel(
 }
 
 // Second kernel: each block follows its link to a word and writes its DXT1
-// block. A link leads to an earlier block, so the walk ends; on the way a block
+// block. A link leads to an earlier block (or is the word that the decoder was made
+// with), so the walk ends; on the way a block
 // replaces its own link (which only it writes) by the one it has just read, so
 // that the blocks behind it skip that part: with all of them walking at once a chain halves
 // at each step, as in pointer jumping, but without a launch and a pass over

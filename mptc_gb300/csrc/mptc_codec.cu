@@ -23,6 +23,7 @@ struct mptc_decoder {
   uint64_t *state = nullptr;  // [ntiles] of the unique blocks' scan, zero between frames; then its tile counter
   uint8_t *planes = nullptr;  // [6][nblk] decoded endpoint planes
   uint32_t *flags = nullptr;  // device error flags, status bits
+  bool state_lost = false;    // a frame's second kernel, which zeroes the state, was not launched
   std::string err;
 };
 
@@ -73,6 +74,10 @@ mptc_status mptc_decoder_create(int32_t width, int32_t height, int32_t search_ar
   if (e == cudaSuccess) e = cudaMalloc(&d->planes, 6 * n);
   if (e == cudaSuccess) e = cudaMalloc(&d->flags, 2 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(d->flags, 0, 2 * sizeof(uint32_t));
+  // every link a word from the start: whatever a block reads leads to a word
+  if (e == cudaSuccess) e = cudaMemset(d->link, 1, n * sizeof(uint64_t));
+  // the memsets are queued, and no other stream's first frame waits for them
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   if (e != cudaSuccess) {
     release(d);
     delete d;
@@ -99,12 +104,18 @@ mptc_status mptc_decode_frame(mptc_decoder *d, const uint8_t *coeff_dev, const u
   cudaStream_t s = (cudaStream_t)stream;
   const int tiles = (d->bw / mptc::kTile) * (d->bh / mptc::kTile);
   uint32_t *claim = reinterpret_cast<uint32_t *>(d->state + d->ntiles);
+  if (d->state_lost) {
+    const cudaError_t z = cudaMemsetAsync(d->state, 0, ((size_t)d->ntiles + 1) * sizeof(uint64_t), s);
+    if (z != cudaSuccess) return dfail(d, MPTC_ECUDA, cudaGetErrorString(z));
+    d->state_lost = false;
+  }
   mptc::launch_after(mptc::decode_parts_kernel, d->ntiles + 6 * tiles, mptc::kCodecThreads, s, coeff_dev, d->bw, d->bh,
                      d->planes, motion_dev, prev_dev, d->sa, unique_dev, n_unique, d->ntiles, d->state, claim, d->link,
                      d->flags, d->flags + 1);
   mptc::launch_chain(mptc::decode_link_kernel, (d->nblk + 255) / 256, 256, s, d->planes, d->nblk, d->link, d->state,
                      d->ntiles, claim, out_dev);
   const cudaError_t e = cudaGetLastError();
+  d->state_lost = e != cudaSuccess;
   return e == cudaSuccess ? MPTC_OK : dfail(d, MPTC_ECUDA, cudaGetErrorString(e));
 }
 
@@ -118,6 +129,7 @@ mptc_status mptc_decoder_check(mptc_decoder *d, void *stream, uint32_t *flags) {
   const uint32_t h = w[0];
   if (flags) *flags = h;
   if (w[1] & mptc::kDevTimeout) return dfail(d, MPTC_ETIMEOUT, "device-side dependency wait expired");
+  if (w[1] & mptc::kDevBadScan) return dfail(d, MPTC_ESTATE, "a frame began before the one before it had ended");
   if (h) {
     std::string m = "decoded frames held";
     if (h & mptc::kDecBadRef) m += " motion codes that copy from outside the frame or from undecoded blocks";
