@@ -45,6 +45,7 @@ struct mptc_ctx {
   int device = 0, sm_count = 0, intra_grid = 0;
   // launch shapes (tunable): warps per CTA of the inter search, CTA cap of the intra search
   int inter_warps = kSearchWarps, intra_cap = 0;
+  int rows_beside = 0;  // CTAs of the row pipeline where other streams' intra frames run too (0: none do)
   // learned proposal (optional): K proposals per block, union rows per
   // scoring stage (4 or 8), bf16 embeddings of this frame's blocks (F) and of
   // the distinct words of the previous frame's final blocks (G, one row per
@@ -376,6 +377,17 @@ int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int g
   return 1;
 }
 
+// CTAs of the row pipeline for one of n frames side by side. Two frames of one CTA per
+// SM each fill the SMs. More are best served one after another, but a narrow frame has
+// no work for that many: a row is some 25 blocks ahead of the next, and the clusters
+// past its rows in flight hold their SMs waiting. Eight 640x360 frames: 1.98 ms with
+// 38 clusters each, 1.37 with 12 (one CTA per block before: 1.79); 256x256: 1.08 and,
+// with 8, 0.54; 1280x720: 4.35 and, with 24, 3.66; from 1920 columns on no difference.
+int rows_ctas_beside(const mptc_ctx *ctx, int n) {
+  if (n <= 2) return ctx->sm_count;
+  return std::min(ctx->sm_count, mptc::kRowCluster * std::max(8, ctx->bw / 13));
+}
+
 // The dynamic shared memory of the row pipeline (its warps' tables) and of the
 // largest window's search.
 cudaError_t search_attrs() {
@@ -685,8 +697,10 @@ mptc_status reencode_finish(mptc_ctx *ctx, const mptc::SearchParams &P, uint32_t
                                            std::min(ctx->nblk, kSweepPartCap), s);
     else
       ctx->launches += launch_intra_frame(P, ctx->order, ig,
-                                          ctx->intra_cap > 0 ? std::min(ctx->intra_cap, ctx->sm_count) : ctx->sm_count,
-                                          ctx->intra_cap <= 0, chained, s);
+                                          ctx->rows_beside > 0 ? ctx->rows_beside
+                                          : ctx->intra_cap > 0 ? std::min(ctx->intra_cap, ctx->sm_count)
+                                                               : ctx->sm_count,
+                                          ctx->rows_beside == 0 && ctx->intra_cap <= 0, chained, s);
   }
   MPTC_CUDA(cudaGetLastError());
   const uint16_t *m16 = P.motion;
@@ -1573,9 +1587,12 @@ mptc_status batch_launch(mptc_batch *b, const int32_t *is_intra, int parity, cud
   if (cudaEventRecord(b->fork_ev, s) != cudaSuccess) return MPTC_ECUDA;
   std::vector<mptc::SearchParams> P(b->n);
   std::vector<LearnedJob> jobs;
+  int n_intra = 0;
+  for (int i = 0; i < b->n; ++i) n_intra += is_intra[i] != 0;
   for (int i = 0; i < b->n; ++i) {
     mptc_ctx *c = b->ctx[i];
     cudaStream_t si = b->streams[i];
+    c->rows_beside = n_intra > 1 && c->intra_cap <= 0 ? rows_ctas_beside(c, n_intra) : 0;  // a cap stands for itself
     if (cudaStreamWaitEvent(si, b->fork_ev, 0) != cudaSuccess) return MPTC_ECUDA;
     const uint64_t *prev = is_intra[i] ? nullptr : b->fin[parity ^ 1][i];
     mptc_status st = mptc_dxt1_encode(c, b->rgb[i], c->stb, c->orig_err, si);
@@ -1654,6 +1671,9 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
                              uint64_t *const *fin, uint8_t *const *mot, uint32_t *const *uni,
                              uint32_t *const *n_uni, cudaStream_t s) {
   const int S = b->n;
+  int lanes = 0;  // with intra frames, all of which are queued at once
+  for (int i = 0; i < S; ++i)
+    lanes += std::any_of(is_intra + (size_t)i * n_frames, is_intra + (size_t)(i + 1) * n_frames, [](int f) { return f; });
   for (int i = 0; i < S; ++i) {
     mptc_ctx *c = b->ctx[i];
     if (!frames[i] || !fin[i] || !mot[i] || !uni[i] || !n_uni[i]) return MPTC_EINVAL;
@@ -1664,7 +1684,9 @@ mptc_status batch_run_frames(mptc_batch *b, int32_t n_frames, const uint8_t *con
     mptc_status st = lane_init(c);
     if (st != MPTC_OK) return st;
     c->lane_b->timing = c->timing;
-    c->lane_b->intra_cap = c->sm_count;  // the lanes share the SMs with each other first (half each: 26.1 ms, not 25.3)
+    // the lanes share the SMs with each other first (half of them each: 26.1 ms, not 25.3)
+    c->lane_b->intra_cap = c->sm_count;
+    c->lane_b->rows_beside = rows_ctas_beside(c, lanes);
     c->lane_b->model = nullptr;  // intra frames: no inter search
     while ((int)b->lane_ev[i].size() < n_frames) {
       cudaEvent_t e;
