@@ -229,7 +229,8 @@ mptc_status mptc_batch_encode_run(mptc_batch *batch, int32_t n_frames, const uin
  * given intra/inter pattern (without advancing the streams) and keeps the
  * fastest: warps (blocks) per CTA of the exhaustive inter search (2, 4; with a
  * model attached the current value is kept), the CTA count of each stream's
- * intra pass (all, 8, 4, 2 or 1 per SM) and, with a model attached, the
+ * intra pass (0: as many as fit, or at most 2, 1, 1/2 or 1/4 per SM; the row
+ * pipeline of an intra frame takes at most 1) and, with a model attached, the
  * dictionary slice per pipeline stage of the window scoring (4 or 8: 64 or
  * 128 words, mptc_ctx_set_learned_shape). Writes the
  * chosen values (any pointer may be NULL; synchronises). The number of

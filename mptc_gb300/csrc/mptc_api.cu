@@ -1982,7 +1982,8 @@ mptc_status mptc_batch_autotune(mptc_batch *b, const int32_t *is_intra, int32_t 
   // trial steps re-encode the current inputs into the buffers of the next
   // real step (same parity), so the streams do not advance. Knobs: warps
   // (blocks) per CTA of the exhaustive inter search, the CTA cap of each
-  // stream's intra dataflow, and, with a model attached, the candidate rows
+  // stream's intra pass (of its sweeps and dataflow, 4 CTAs per SM without one, and
+  // of the row pipeline, at most 1), and, with a model attached, the candidate rows
   // (dictionary slice) per pipeline stage of the window scoring.
   const bool learned = b->ctx[0]->model != nullptr;
   std::vector<int> warps = {2, 4}, rows = {8};
@@ -1991,7 +1992,7 @@ mptc_status mptc_batch_autotune(mptc_batch *b, const int32_t *is_intra, int32_t 
     rows = {4, 8};
   }
   const int sms = b->ctx[0]->sm_count;
-  const int caps[5] = {0, 8 * sms, 4 * sms, 2 * sms, sms};
+  const int caps[5] = {0, 2 * sms, sms, sms / 2, sms / 4};
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return MPTC_ECUDA;
   float best = 1e30f;
