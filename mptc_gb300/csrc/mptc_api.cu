@@ -349,9 +349,20 @@ constexpr int kRowsAlone = 120 * 1024;
 static_assert(2 * (sizeof(mptc::RowShared) + 1024) <= 228 * 1024 && sizeof(mptc::RowShared) <= kRowsAlone,
               "two CTAs of the row pipeline share an SM");
 
+// A frame by itself takes one CTA of the row pipeline per SM up to this many block
+// columns, two from there on. The more columns, the more rows are in flight, and past
+// some 25 of them it is not the chain that bounds the frame but its blocks' workers,
+// of which two CTAs hold twice as many. One CTA | two per SM, in us, sa 1, 2 and 8:
+// 1920x1080 939 | 743, 1176 | 1268, 1524 | 1747; 2560x1440 1592 | 1180, 2016 | 1941,
+// 2359 | 2348; 3840x2160 3383 | 2393, 4305 | 3662, 4836 | 3841; 3840x360 718 | 591,
+// 893 | 846, 1119 | 1085. (The dataflow before took 4118 at 3840x2160 and sa 2.) A
+// frame of no more rows than the clusters of one CTA per SM gives each its own row
+// (65536x16, sa 2: 4328 | 5401).
+constexpr int kRowsWide = 640;
+
 // The intra search of a whole intra frame, behind launch_begin: the row pipeline
-// with `ctas` CTAs at sa <= 8 (alone: one per SM; otherwise beside other frames, two
-// per SM), the block dataflow on `grid` CTAs for larger windows.
+// with `ctas` CTAs at sa <= 8 (beside other frames; alone: with `ctas` or twice as
+// many, see kRowsWide), the block dataflow on `grid` CTAs for larger windows.
 // Returns the number of kernels launched.
 int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int grid, int ctas, bool alone,
                        bool chained, cudaStream_t s) {
@@ -359,6 +370,10 @@ int launch_intra_frame(const mptc::SearchParams &P, const uint32_t *order, int g
   if (P.sa > 8) {
     mptc::intra_search_kernel<kIntraThreads><<<grid, kIntraThreads, 0, s>>>(P, order, nullptr, nblk);
     return 1;
+  }
+  if (alone && P.bw >= kRowsWide && P.bh > ctas / mptc::kRowCluster) {
+    alone = false;
+    ctas *= 2;
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(mptc::kRowCluster * std::max(1, std::min(P.bh, ctas / mptc::kRowCluster)));

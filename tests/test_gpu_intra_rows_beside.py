@@ -1,7 +1,8 @@
-"""The row pipeline with two CTAs per SM (intra_rows_kernel<2>), which runs the intra
-frames of several streams side by side: batches of two, and of three and more streams,
-whose frames take fewer clusters the narrower they are, as a run and step by step,
-against the oracle."""
+"""The row pipeline with two CTAs per SM (intra_rows_kernel<2>) against the oracle. It
+runs the intra frames of several streams side by side: batches of two, and of three and
+more streams, whose frames take fewer clusters the narrower they are, as a run and step
+by step. And frames by themselves from 640 block columns and 39 block
+rows on."""
 import numpy as np
 import pytest
 
@@ -45,3 +46,23 @@ def test_frames_side_by_side_match_oracle(sizes, sa, kind):
             np.testing.assert_array_equal(uni, r.unique)
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("w,h,sa,kind", [(2556, 160, 8, "mixed"), (2560, 152, 8, "mixed"), (2560, 156, 8, "noise"),
+                                         (2564, 340, 1, "stream"), (3840, 200, 2, "mixed")])
+def test_wide_frames_match_oracle(w, h, sa, kind):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from mptc_gb300.encoder import Encoder
+    f = frame(kind, w, h, seed=w + h + sa)
+    ref = oracle.encode_stream(f[None], sa, 5, 16, threads=8)[0]
+    enc = Encoder(w, h, sa, 5, 16)
+    try:
+        for _ in range(2):
+            out = enc.encode_frame_host(f, is_intra=True)
+            np.testing.assert_array_equal(out.final, ref.final)
+            np.testing.assert_array_equal(out.motion, ref.motion)
+            np.testing.assert_array_equal(out.unique, ref.unique)
+    finally:
+        enc.close()
