@@ -229,8 +229,12 @@ __global__ void __launch_bounds__(THREADS, 4) intra_search_kernel(SearchParams P
 // open. So where the first sweep has changed more than a third of the open
 // blocks, or the second more than a third of what the first has, the rest are
 // skipped: a 1280x720 frame after a cut takes 990 us instead of 1,531, of which six
-// vain sweeps were 725, a 1080p one 2,090 instead of 3,782. Few changes (up to 8)
-// fall unevenly and are left to the sweeps.
+// vain sweeps were 725, a 1080p one 2,090 instead of 3,782. Few changes fall unevenly
+// (74, 28, 11, 5, 0) and the sweeps that follow them are cheap beside the dataflow of
+// all open blocks: up to a sixteenth of these (and 8) are left to the sweeps. 656 frames of
+// cuts, scrolls, fades, noise and changed parts: without that bound 2 of the 47 given up
+// by their second sweep would have converged (282 us instead of 87, 506 instead of 156);
+// with it none, and 12 that now take all sweeps in vain lose 2 to 8% (550 | 573 us).
 constexpr uint32_t kSweepGivenUp = 0xFFFFFFFFu;
 
 // Inter frames: the intra search of the blocks the inter pass left open, as
@@ -275,8 +279,9 @@ __global__ void __launch_bounds__(THREADS, 3) intra_sweep_kernel(SearchParams P,
   depend();
   release_next();
   // loaded together: one latency
-  const uint32_t changed = __ldcg(changed_in), limit = changed_before ? __ldcg(changed_before) / 3u : ~0u - 1u;
+  const uint32_t changed = __ldcg(changed_in), earlier = changed_before ? __ldcg(changed_before) : 0u;
   const int n_pend = (int)__ldcg(n_pending_dev);
+  const uint32_t limit = changed_before ? max(earlier / 3u, (uint32_t)n_pend / 16u) : ~0u - 1u;
   int idx = (int)__ldcg(pending + min((int)blockIdx.x, P.bw * P.bh - 1));  // unused where there is none
   if (changed == 0u) return;
   if (changed > max(limit, 8u)) {  // uniform over the grid; a sweep given up before is above any limit
