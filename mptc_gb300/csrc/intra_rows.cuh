@@ -118,18 +118,21 @@ struct __align__(16) RowWork {
   uint32_t eps[kRowBuckets];  // its endpoints
   uint16_t list[kRowBuckets];
 };
-// What the chain needs of a block, and its answer (base and word tagged with the
-// group; base's half is written last and read first).
+// What the chain needs of a block, and its answer. The chain and the workers read
+// each other's words while they are written, without a fence on the chain's path:
+// every 64-bit half of a vector is written and read whole, is complete by itself and
+// carries the group's tag in its top bits, so it does not matter in which order
+// they are seen. The tables' entries are as complete (a word and its err_diff); the
+// chain reads them behind the barrier that follows their reset (group_ready).
 struct __align__(16) RowMail {
   uint64_t base;       // the word selected without the left neighbours, or the block's own
   uint32_t wins;       // (max(err_diff, 0) << 5 | lane) below which a left neighbour wins
-  uint32_t pos;        // position of base (kNoMatch: not accepted), that of later << 16
+  uint32_t pos;        // position of base (kNoMatch: not accepted), that of later << 16, tag
   uint64_t later;      // the word of the last row's err_diff < 0: an err_diff <= 0 gives way to it
   uint32_t own;
-  uint32_t gives;      // 32 if there is such a word, else 0
-  uint64_t word;       // the chain's answer: the final word,
-  uint32_t wpos;       // its position (kNoMatch: not accepted)
-  uint32_t pad;
+  uint32_t gives;      // 32 if there is such a word, else 0; tag
+  uint64_t word;       // the chain's answer: the final word, for the blocks to its right;
+  uint64_t answer;     // its index word and, above it, its position (kNoMatch: not accepted), for the worker
 };
 struct RowShared {
   RowDict dict;
@@ -153,18 +156,18 @@ __device__ __forceinline__ T ld_volatile(const T *p) {
   return *reinterpret_cast<const volatile T *>(p);
 }
 
-__device__ __forceinline__ uint4 ld_shared_v4(const void *p) {
-  uint4 v;
-  asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+// Two adjacent 64-bit words, each read or written whole: x, y and z, w.
+__device__ __forceinline__ uint4 ld_shared_2x64(const void *p) {
+  uint64_t a, b;
+  asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];"
+               : "=l"(a), "=l"(b)
                : "r"((uint32_t)__cvta_generic_to_shared(p))
                : "memory");
-  return v;
+  return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
 }
-
-__device__ __forceinline__ void st_shared_v4(void *p, uint4 v) {
-  asm volatile("st.volatile.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"((uint32_t)__cvta_generic_to_shared(p)),
-               "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+__device__ __forceinline__ void st_shared_2x64(void *p, uint4 v) {
+  asm volatile("st.volatile.shared.v2.u64 [%0], {%1, %2};" ::"r"((uint32_t)__cvta_generic_to_shared(p)),
+               "l"((uint64_t)v.y << 32 | v.x), "l"((uint64_t)v.w << 32 | v.z)
                : "memory");
 }
 
@@ -269,6 +272,18 @@ __device__ __forceinline__ void worker_barrier() {
   asm volatile("bar.sync 1, %0;" ::"n"(32 * kRowGroup) : "memory");
 }
 
+// The group's tables are reset and its blocks staged: worker 0 behind a barrier of all
+// workers, to the chain. A worker gets there whether or not its waits gave up, and the
+// chain asks once for each of its groups.
+__device__ __forceinline__ void group_ready() {
+  __syncwarp();
+  asm volatile("bar.arrive 2, 64;" ::: "memory");
+}
+__device__ __forceinline__ void await_group() {
+  __syncwarp();
+  asm volatile("bar.sync 2, 64;" ::: "memory");
+}
+
 // One group's block by worker k (see above): steps A to C, then the answer
 // written out.
 __device__ __forceinline__ void row_worker(RowShared &S, const SearchParams &P, int k, int g, int by, int lane) {
@@ -308,6 +323,7 @@ __device__ __forceinline__ void row_worker(RowShared &S, const SearchParams &P, 
     if (t == 0) D.count = 0;
   }
   worker_barrier();
+  if (k == 0) group_ready();
   // rounds 0-11: a row of the union each, y-4 .. y-15; 12: the stb words of
   // row y-1; 13: those of the left neighbours in row y and of the group itself
   const int u0 = x0 - sa - kRowBack, nu = 2 * sa + kRowGroup - 1 + kRowBack;  // the union's columns
@@ -456,16 +472,18 @@ __device__ __forceinline__ void row_worker(RowShared &S, const SearchParams &P, 
   if (lane == 0) {
     __threadfence_block();
     const uint64_t bt = base | tag;
+    const uint32_t hi = (uint32_t)(tag >> 32);
     // err_diffs are at most 65025
     const uint32_t wins = thr < 0 ? 0u : (uint32_t)(min(le0 ? 0 : min_e, min(thr, 65535)) + 1) << 5;
-    st_shared_v4(&M.later, make_uint4((uint32_t)later, (uint32_t)(later >> 32), own, neg >= 0 && thr >= 0 ? 32u : 0u));
-    st_shared_v4(&M.base, make_uint4((uint32_t)bt, (uint32_t)(bt >> 32), wins,
-                                     (pos < 0 ? kNoMatch : (uint32_t)pos) | ((uint32_t)later_pos << 16)));
+    st_shared_2x64(&M.later, make_uint4((uint32_t)later, (uint32_t)(later >> 32) | hi, own,
+                                        (neg >= 0 && thr >= 0 ? 32u : 0u) | hi));
+    st_shared_2x64(&M.base, make_uint4((uint32_t)bt, (uint32_t)(bt >> 32), wins,
+                                     (pos < 0 ? kNoMatch : (uint32_t)pos) | ((uint32_t)later_pos << 16) | hi));
   }
   // Until the chain answers, the left neighbours' words are evaluated as they
   // appear: lane d - 1 watches the neighbour at distance d, in its mail or,
   // before the group, among the words handed over.
-  uint4 ans = make_uint4(0u, 0u, 0u, 0u);
+  uint64_t ans = 0;
   {
     bool open = lane < sa && lane > 0 && bx > lane;
     const uint64_t *src = lane < k ? &S.mail[k - 1 - lane].word : S.hist + ((lane - k) & 7);
@@ -476,19 +494,19 @@ __device__ __forceinline__ void row_worker(RowShared &S, const SearchParams &P, 
         l = ld_volatile(src);
         if (((uint32_t)(l >> 32) ^ hi) >> 27) l = 0;
       }
-      ans = ld_shared_v4(&M.word);
+      ans = ld_volatile(&M.answer);
       if (__any_sync(kFull, l != 0ull)) {
         if (l != 0ull) open = false;
         row_value(S, D, W, P, pg, l & kRowWord, own, orig, sumsq);
       }
-      if (!__any_sync(kFull, ((ans.y ^ hi) >> 27) != 0u) || dead) break;
+      if (!__any_sync(kFull, (((uint32_t)(ans >> 32) ^ hi) >> 27) != 0u) || dead) break;
       __nanosleep(40);
       dead = limit.warp_over(P.status);
     }
   }
   __threadfence_block();
   if (lane == 0) {
-    const uint32_t p = ans.z, word = ans.x;
+    const uint32_t p = (uint32_t)(ans >> 32) & 0x1FFu, word = (uint32_t)ans;
     uint64_t blk = stb;
     if (p != kNoMatch && word != own) {
       uint32_t b = row_hash(word);
@@ -532,8 +550,8 @@ __device__ __noinline__ RowAnswer row_decide(RowShared &S, const SearchParams &P
                      ld_volatile(&Wl.sumsq));
       }
     }
-    __threadfence_block();
     __syncwarp();
+    __threadfence_block();  // before lane 0's answer, behind which the workers read
     v = __shfl_sync(kFull, v, 0);
     if (lane == l) e = v;
   }
@@ -548,8 +566,8 @@ __device__ __noinline__ RowAnswer row_decide(RowShared &S, const SearchParams &P
     r.word = (((uint64_t)ma.y << 32) | ma.x) & kRowWord;
     r.pos = ma.w & 0x1FFu;
   }
-  if (m < mb.w) {
-    r.word = ((uint64_t)mb.y << 32) | mb.x;
+  if (m < (mb.w & 32u)) {
+    r.word = (((uint64_t)mb.y << 32) | mb.x) & kRowWord;
     r.pos = (ma.w >> 16) & 255u;
   }
   return r;
@@ -570,7 +588,7 @@ __global__ void __launch_bounds__(kRowThreads, PER_SM) intra_rows_kernel(SearchP
   const uint32_t next_hist = cluster_map(S.hist, (rank + 1u) % ncta);
   for (;;) {
     cluster_sync();  // the previous row is decided
-    if (tid < kRowGroup) S.mail[tid].base = S.mail[tid].word = 0;
+    if (tid < kRowGroup) S.mail[tid] = RowMail{};
     if (tid < 8) S.hist[tid] = 0;
     if (rank == 0 && tid == 0) {
       const uint32_t y = atomicAdd(P.work, 1u);
@@ -589,6 +607,7 @@ __global__ void __launch_bounds__(kRowThreads, PER_SM) intra_rows_kernel(SearchP
       uint64_t h = 0;
 #pragma unroll 1
       for (int g = (int)rank; g < groups; g += (int)ncta) {
+        await_group();
         if (g > 0 && ncta > 1) {
           const uint32_t tag = (uint32_t)(row_tag(g) >> 59);
           WaitLimit limit;
@@ -606,26 +625,27 @@ __global__ void __launch_bounds__(kRowThreads, PER_SM) intra_rows_kernel(SearchP
         // nearest, which is the first in scan order. The lanes of one load need not see the same
         // store, so they decide together.
         const uint32_t tag = (uint32_t)(row_tag(g) >> 32);
+        uint32_t hlo = (uint32_t)h, hhi = (uint32_t)(h >> 32);  // h in halves
         const int nb = min(kRowGroup, bw - g * kRowGroup);
         const RowWork *W = S.w;
         RowMail *M = S.mail;
         uint64_t *done = P.done + (size_t)by * bw + g * kRowGroup;
 #pragma unroll 1
         for (int k = 0; k < nb && !dead; ++k, ++W, ++M, ++done) {
-          const uint32_t lo = (uint32_t)h, hi = (uint32_t)(h >> 32), hb = row_hash(lo);
+          const uint32_t lo = hlo, hi = hhi, hb = row_hash(lo);
           const bool on = hi != 0u && lane < sa;
           uint4 ma, mb;
           uint32_t m;
           bool slow;
           WaitLimit limit;
           for (;;) {  // until the block's mail is there
-            ma = ld_shared_v4(&M->base);
-            mb = ld_shared_v4(&M->later);
+            ma = ld_shared_2x64(&M->base);
+            mb = ld_shared_2x64(&M->later);
             unsigned long long v = ld_volatile(reinterpret_cast<const unsigned long long *>(&W->ent[hb]));
             const unsigned long long v2 = ld_volatile(
                 reinterpret_cast<const unsigned long long *>(&W->ent[row_after(hb)]));
             if ((uint32_t)v != lo) v = v2;
-            const bool wait = ((tag ^ ma.y) >> 27) != 0u;
+            const bool wait = ((tag ^ ma.y) | (tag ^ ma.w) | (tag ^ mb.y) | (tag ^ mb.w)) >= 1u << 27;
             m = __reduce_min_sync(kFull, on ? ((uint32_t)max((int)(v >> 32), 0) << 5) | (uint32_t)lane : 0xFFFFFFFFu);
             slow = __any_sync(kFull, wait || (on && (uint32_t)v != lo));
             if (!slow || !__any_sync(kFull, wait)) break;
@@ -633,30 +653,34 @@ __global__ void __launch_bounds__(kRowThreads, PER_SM) intra_rows_kernel(SearchP
             if (dead) break;
           }
           if (dead) break;  // the workers' waits give up too
-          // the words move one lane up; lane 0 takes the block's
-          const uint64_t hn = __shfl_sync(kFull, h, lane == 0 ? (int)(m & 31u) : lane - 1);
-          uint64_t w = hn;
-          uint32_t pos = (uint32_t)sa + (m & 31u);
+          // the words move one lane up; lane 0 takes the block's (whi and pos with the tag)
+          const int from = lane == 0 ? (int)(m & 31u) : lane - 1;
+          const uint32_t nlo = __shfl_sync(kFull, lo, from), nhi = __shfl_sync(kFull, hi, from);
+          uint32_t wlo = nlo, whi = nhi | tag;
+          uint32_t pos = tag + (uint32_t)sa + (m & 31u);
           if (m >= ma.z) {
-            w = ((uint64_t)(ma.y & 0x07FFFFFFu) << 32) | ma.x;
-            pos = ma.w & 0x1FFu;
+            wlo = ma.x, whi = ma.y;
+            pos = ma.w & 0xF80001FFu;
           }
-          if (m < mb.w) {
-            w = ((uint64_t)mb.y << 32) | mb.x;
-            pos = ma.w >> 16;
+          if (m < (mb.w & 32u)) {
+            wlo = mb.x, whi = mb.y;
+            pos = tag | (ma.w >> 16 & 255u);
           }
           if (slow) {
-            const RowAnswer r = row_decide(S, P, k, nb, h, ma, mb, lane);
-            w = r.word;
-            pos = r.pos;
+            const RowAnswer r = row_decide(S, P, k, nb, (uint64_t)hhi << 32 | hlo, ma, mb, lane);
+            wlo = (uint32_t)r.word, whi = (uint32_t)(r.word >> 32) | tag;
+            pos = r.pos | tag;
           }
-          h = lane == 0 ? w : hn;
+          const uint32_t wsrc = whi & 0x07FFFFFFu;
+          hlo = lane == 0 ? wlo : nlo;
+          hhi = lane == 0 ? wsrc : nhi;
           if (lane == 0) {
-            st_relaxed(done, w);
-            st_shared_v4(&M->word, make_uint4((uint32_t)w, (uint32_t)(w >> 32) | tag, pos, 0u));
+            st_relaxed(done, (uint64_t)wsrc << 32 | wlo);
+            st_shared_2x64(&M->word, make_uint4(wlo, whi, wlo, pos));
           }
           __syncwarp();
         }
+        h = (uint64_t)hhi << 32 | hlo;
         if (lane < 8 && g + 1 < groups && ncta > 1)
           st_cluster(next_hist + 8u * (uint32_t)lane, h | row_tag(g + 1));
       }
