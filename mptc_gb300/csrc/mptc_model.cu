@@ -421,8 +421,12 @@ mptc_status mptc_model_create(uint64_t seed, mptc_model **out) {
     mptc_model_destroy(m);
     return st;
   }
-  cudaMemset(m->m, 0, n * sizeof(float));
-  cudaMemset(m->v, 0, n * sizeof(float));
+  // the moments are zero before any other stream's first step reads them
+  if (cudaMemset(m->m, 0, n * sizeof(float)) != cudaSuccess || cudaMemset(m->v, 0, n * sizeof(float)) != cudaSuccess ||
+      cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    mptc_model_destroy(m);
+    return MPTC_ECUDA;
+  }
   *out = m;
   return MPTC_OK;
 }
