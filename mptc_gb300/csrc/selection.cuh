@@ -1,6 +1,6 @@
-// The reference's selection rule over a search window in closed form, for a
-// warp (LaneSel, warp_select) and for a CTA (ThreadSel, CtaReduce,
-// cta_select), and the parameters every search kernel takes.
+// The reference's selection rule over a search window in closed form, for a CTA
+// whose threads hold its positions (LaneSel, ThreadSel, CtaReduce, cta_select), and the
+// parameters every search kernel takes.
 #pragma once
 #include <cstdint>
 
@@ -8,9 +8,8 @@
 
 namespace mptc {
 
-// The selection rule in closed form, for a warp that holds all positions of
-// a window spread over its lanes (each lane visits its positions in scan
-// order). The reference loop (if e < m { m = e; sel = pos; if e <= 0 { m = 0;
+// The selection rule in closed form, for threads that hold the positions of a window
+// between them. The reference loop (if e < m { m = e; sel = pos; if e <= 0 { m = 0;
 // break the row } }) selects:
 // - if some valid position has e <= 0: let P0 be the first (scan order) and
 //   r0 its row. Later rows replace the selection with their first e < 0 (e < 0
@@ -18,10 +17,10 @@ namespace mptc {
 //   e < 0 gives its first e < 0; without one the selection stays P0. Rows
 //   before r0 hold no e <= 0, and row r0 breaks at P0. m = 0.
 // - otherwise the first position of the minimum e (strict improvement), m = it.
-// Each lane keeps the three positions (first e <= 0; the key
+// Each thread keeps the three positions (first e <= 0; the key
 // row << 16 | (0xFFFF - pos) of its e < 0 positions; first minimum, ties
-// broken by position, so a lane may visit its positions in any order); four
-// warp reductions give the selected position, whose candidate data the caller
+// broken by position, so a thread may visit its positions in any order); reductions
+// over the threads give the selected position, whose candidate data the caller
 // recovers.
 struct LaneSel {
   int le0_pos = 0x7fffffff;  // first position with e <= 0
@@ -37,19 +36,6 @@ struct LaneSel {
     }
   }
 };
-
-// Returns the selected position (-1 when no position is valid) and its m.
-__device__ __forceinline__ int warp_select(const LaneSel &l, int w2, int &m) {
-  const int p0 = __reduce_min_sync(kFull, l.le0_pos);
-  if (p0 != 0x7fffffff) {
-    m = 0;
-    const int key = __reduce_max_sync(kFull, l.neg_key);
-    return (key >= 0 && (key >> 16) > p0 / w2) ? 0xFFFF - (key & 0xFFFF) : p0;
-  }
-  m = __reduce_min_sync(kFull, l.min_e);
-  const int p = __reduce_min_sync(kFull, l.min_e == m ? l.min_pos : 0x7fffffff);
-  return p == 0x7fffffff ? -1 : p;
-}
 
 // The same closed form for a CTA whose threads each hold positions base + tid
 // of successive rounds, keeping for each of the three statistics the
@@ -131,13 +117,13 @@ __device__ __forceinline__ uint64_t done_word(uint64_t blk) { return (1ull << 32
 
 struct SearchParams {
   const uint8_t *rgb;
-  const float4 *wdesc;    // weight sums of the previous frame's final blocks (inter)
+  const float4 *wdesc;    // weight sums of the previous frame's final blocks (inter), of the stb blocks (row pipeline)
   const uint64_t *stb;
   const int32_t *orig_err;
   const uint64_t *prev;   // previous frame's final blocks (inter)
   uint64_t *final_blk;
   uint16_t *motion;       // (x | y << 8) per block
-  uint64_t *done;         // per block: 0 while open, done_word(final block) once final
+  uint64_t *done;         // per block: 0 while open, done_word(final block) once final (done_src in the row pipeline)
   uint32_t *work;         // dataflow work counter
   uint32_t *status;       // device status bits
   int width, bw, bh, sa, thr;
