@@ -44,7 +44,7 @@ C_CAND, C_DXT = 600, 1500
 # DRAM bytes (read + write) per launch of the search kernels on the 1080p
 # stream, from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum);
 # the summaries under profiles/ give the commands.
-NCU_TRAFFIC = {"inter_search": 10_925_312, "intra_search_kernel": 10_824_192 + 86_272}
+NCU_TRAFFIC = {"inter_search": 10_925_312, "intra_search_kernel": 10_822_912 + 82_944}
 
 
 def algo_bytes(kernel: str, n: int) -> int:

@@ -39,11 +39,11 @@ namespace mptc {
 // inter_overflow_kernel searches afterwards with a CTA per block: those runs
 // cost several times a smooth one and, kept in one warp, would hold their SM
 // long after the other warps finished.
-// Bound by issue (84% of the slots), 927 warp instructions a block on the 1080p
-// test stream: evaluation 272 (73 of them the test for a near tie), deduplication
-// 194, lists 89, selection 67, the exact passes 130, the rest staging. 132 us a
-// frame, against 226 (1,566 instructions) with each block's words evaluated by
-// themselves from a table of float products in shared memory.
+// Bound by issue (80% of the slots), 846 warp instructions a block on the 1080p
+// test stream: evaluation about 255, deduplication 194, lists 89, selection 67, the
+// exact refits about 70, the rest staging. 122 us a frame, against 226 (1,566
+// instructions) with each block's words evaluated by themselves from a table of
+// float products in shared memory.
 constexpr int kRun = 8;
 constexpr int kRunWords = 128;  // distinct union words handled by the run table
 constexpr int kRunBuckets = 256;
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
 // A union of more distinct words than the table takes (noise) is searched in
 // slabs of rows that fit it, whose selections are merged.
 // A warp per block and a table per span of 256 positions before: 510 us for an
-// 856x480 frame at sa 24, under 200 now (the whole frame 302, before 642).
+// 856x480 frame at sa 24, 184 now (the whole frame 306, before 690).
 constexpr int kWideThreads = 256, kWideBuckets = 1024, kWideWords = 640;
 // The buckets' table is never full: a thread inserts only after it has read a
 // count of at most kWideWords, and counts each word before its next.

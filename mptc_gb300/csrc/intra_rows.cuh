@@ -76,13 +76,16 @@ __device__ __forceinline__ uint64_t ld_shared_relaxed(const uint64_t *p) {
 // streams up to 2560x1440 and their 15 learned inter frames take 25.3 ms, with one 27.9.
 //
 // Bound by latency: the critical path of an intra frame is bw + sa * bh steps
-// from a block to its right neighbour or to the row below, here about 0.2 us
-// and 1 us, with one warp's chains of dependent instructions (about 5 cycles
-// each) on them. So whatever can be known before the last neighbour is taken
-// off that path, and a row's work is spread over four SMs. 1920x1080: 1.54 ms,
-// 256x256: 0.30 ms, against 3.64 and 0.80 ms with one CTA per block polling
-// global memory (intra_search_kernel); clusters of 2, 3, 5 and 6 CTAs: 2.2, 1.77,
-// 1.54, 1.9 ms at 1080p; two sets of workers per CTA: 1.8 ms.
+// from a block to its right neighbour or to the row below, with one warp's chains of
+// dependent instructions (about 5 cycles each) on them. So whatever can be known
+// before the last neighbour is taken off that path, and a row's work is spread over
+// four SMs. Clock stamps at 1080p and sa 8: a block takes the chain some 680 cycles,
+// 320 of instructions, as many waiting for its mail (every fourth block) and 35 in
+// row_decide (every 30th); a row takes 190 us and follows the one above by 5.3 us, so
+// that 36 rows are in flight, about as many as there are clusters. A 1080p frame 1.43 to
+// 1.52 ms, a 256x256 one 0.28 to 0.32, against 3.66 and 0.86 with one CTA per block polling
+// global memory (intra_search_kernel). When it took 1.54 ms, clusters of 2, 3, 5 and
+// 6 CTAs took 2.2, 1.77, 1.54 and 1.9, two sets of workers per CTA 1.8.
 constexpr int kRowCluster = 4;  // CTAs per row
 constexpr int kRowGroup = 8;    // blocks per group, worker warps per CTA
 constexpr int kRowThreads = 32 * (kRowGroup + 1);
@@ -574,8 +577,9 @@ __device__ __noinline__ RowAnswer row_decide(RowShared &S, const SearchParams &P
 }
 
 // PER_SM: CTAs that an SM holds at once. A frame by itself is fastest with one (two
-// of its CTAs on an SM slow the chain: 1.81 ms against 1.51 at 1080p); frames
-// beside others' take half the registers and share the SMs.
+// of its CTAs on an SM slow the chain: 1.75 ms against 1.52 at 1080p), unless it is wide;
+// wide frames and frames beside others' take half the registers and share the SMs
+// (launch_intra_frame has the rule).
 template <int PER_SM>
 __global__ void __launch_bounds__(kRowThreads, PER_SM) intra_rows_kernel(SearchParams P) {
   extern __shared__ __align__(16) uint8_t row_smem[];

@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1) score_topk_tc_kernel(const _
 // would. Results are 16-bit ranks (run_rank) and endpoints per block and
 // proposal; then lane = block selects. Bound by issue. With a table of float
 // products per block, the proposals of 32/K blocks per warp and the selection by
-// shuffles it took 44 us for a 1080p frame's 8 proposals a block, 29 now.
+// shuffles it took 46 us for a 1080p frame's 8 proposals a block, 27 now.
 // The frames of up to kMaxBatch jobs per launch: job j owns the block groups
 // [group_end[j-1], group_end[j]) of `group` blocks each.
 constexpr int kEvalWarps = 4, kEvalGroup = 32;
