@@ -43,7 +43,8 @@ W, H, FRAMES, SA, THR, II = 1920, 1080, 120, 8, 5, 16
 C_CAND, C_DXT = 600, 1500
 # DRAM bytes (read + write) per launch of the search kernels on the 1080p
 # stream, from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum);
-# the summaries under profiles/ give the commands.
+# the summaries under profiles/ give the commands. The timers report the row
+# pipeline of an intra frame (intra_rows_kernel) as intra_search_kernel.
 NCU_TRAFFIC = {"inter_search": 10_925_312, "intra_search_kernel": 10_822_912 + 82_944}
 
 

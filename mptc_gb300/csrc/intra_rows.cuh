@@ -146,7 +146,9 @@ struct RowShared {
   uint8_t snap5[256], snap6[256];
 };
 
-static_assert(sizeof(RowDict) % 16 == 0 && offsetof(RowWork, ent) % 16 == 0 && offsetof(RowMail, later) % 16 == 0, "vector stores reset the tables");
+static_assert(sizeof(RowDict) % 16 == 0 && offsetof(RowWork, ent) % 16 == 0 && offsetof(RowMail, later) % 16 == 0 &&
+                  offsetof(RowMail, word) % 16 == 0,
+              "vector accesses of the tables and the mail");
 
 __device__ __forceinline__ uint32_t row_hash(uint32_t w) {
   return __umulhi(w * 2654435761u, (uint32_t)kRowBuckets);

@@ -236,7 +236,8 @@ enum KernelId {
 };
 // inter_search: the inter search kernels of an inter frame (inter_run_kernel
 // and inter_overflow_kernel at sa <= 8, inter_wide_kernel above; the
-// learned proposal's kernels when a model is attached)
+// learned proposal's kernels when a model is attached). intra_search_kernel: the
+// intra search of an intra frame, intra_rows_kernel at sa <= 8
 const char *kKernelNames[K_COUNT] = {"dxt1_encode_kernel",      "inter_search",
                                      "intra_search_kernel",     "intra_sweep_kernel/inter_frame",
                                      "unique_scan_kernel",      "word_dict+embed_kernel/g",
